@@ -38,6 +38,14 @@ cudaError_t launch_dispatch_tiny(const DispatchArgs& a, bool send, bool recv, in
 cudaError_t launch_dispatch_tiny_multi(const DispatchMulti& args, int nranks, bool send, bool recv,
                                        int grid, cudaStream_t stream);
 
+// Objects whose world is one rank (single_rank.cu): dispatch as one call or as halves, the packed
+// send (a.packed), and combine as one call.  `limit`: blocks at most.
+size_t single_rank_smem_bytes(const A2AParams& p);
+cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, int limit,
+                                   cudaStream_t stream);
+cudaError_t launch_single_combine(const CombineArgs& a, DType in, DType out, int limit,
+                                  cudaStream_t stream);
+
 size_t combine_smem_bytes(const A2AParams& p);
 int combine_threads();
 

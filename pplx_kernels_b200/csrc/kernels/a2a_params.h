@@ -42,6 +42,7 @@
 namespace pplx {
 
 constexpr int kMaxWorld = 16;
+constexpr uint32_t kNoRow = 0xffffffffu;
 
 struct A2AParams {
   // geometry
@@ -100,6 +101,9 @@ struct A2AParams {
   uint32_t* comb_iter;    // number of dispatches started = ordinal of the coming combine
   uint32_t* recv_count;   // [nle] rows received per local expert by the last dispatch
   uint2* row_src;         // [nle][cap] {src_rank | k << 16, src_token} per received row
+  uint2* row_of;          // world of one rank: [max_tokens * topk] {local expert, row} of every
+                          //     (token, k) of the last dispatch, {kNoRow, 0} where it has none;
+                          //     nullptr otherwise
   Status* status;
   uint64_t timeout_ns;
   uint64_t* trace;        // optional [kTraceSlots] %globaltimer stamps of block 0, or null

@@ -46,6 +46,7 @@
 #include "a2a_device.cuh"
 #include "a2a_kernels.h"
 #include "a2a_params.h"
+#include "combine_device.cuh"
 
 namespace pplx {
 namespace {
@@ -90,106 +91,40 @@ __device__ __forceinline__ void trace_block(const A2AParams& p, int first_slot) 
     p.trace[first_slot + blockIdx.x] = ptx::globaltimer_ns();
 }
 
-// ---- 8-element vector helpers ------------------------------------------------
-
-template <typename T>
-struct Vec8;
-
-template <>
-struct Vec8<float> {
-  int4 a, b;
-  __device__ __forceinline__ void load_cg(const void* p) {
-    a = ptx::ld_cg_v4(p);
-    b = ptx::ld_cg_v4(static_cast<const uint8_t*>(p) + 16);
-  }
-  __device__ __forceinline__ void fma_into(float (&acc)[8], float w) const {
-    acc[0] = fmaf(w, __int_as_float(a.x), acc[0]);
-    acc[1] = fmaf(w, __int_as_float(a.y), acc[1]);
-    acc[2] = fmaf(w, __int_as_float(a.z), acc[2]);
-    acc[3] = fmaf(w, __int_as_float(a.w), acc[3]);
-    acc[4] = fmaf(w, __int_as_float(b.x), acc[4]);
-    acc[5] = fmaf(w, __int_as_float(b.y), acc[5]);
-    acc[6] = fmaf(w, __int_as_float(b.z), acc[6]);
-    acc[7] = fmaf(w, __int_as_float(b.w), acc[7]);
-  }
-};
-
-__device__ __forceinline__ float2 unpack2(__half2 h) { return __half22float2(h); }
-__device__ __forceinline__ float2 unpack2(__nv_bfloat162 h) { return __bfloat1622float2(h); }
-
-template <typename T2>
-struct Vec8Half {
-  int4 a;
-  __device__ __forceinline__ void load_cg(const void* p) { a = ptx::ld_cg_v4(p); }
-  __device__ __forceinline__ void fma_into(float (&acc)[8], float w) const {
-    const T2* h = reinterpret_cast<const T2*>(&a);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = unpack2(h[j]);
-      acc[2 * j] = fmaf(w, f.x, acc[2 * j]);
-      acc[2 * j + 1] = fmaf(w, f.y, acc[2 * j + 1]);
-    }
-  }
-};
-template <>
-struct Vec8<__half> : Vec8Half<__half2> {};
-template <>
-struct Vec8<__nv_bfloat16> : Vec8Half<__nv_bfloat162> {};
-
-__device__ __forceinline__ int4 pack8(const float (&acc)[8], __half*) {
-  int4 r;
-  __half2* h = reinterpret_cast<__half2*>(&r);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) h[j] = __floats2half2_rn(acc[2 * j], acc[2 * j + 1]);
-  return r;
-}
-__device__ __forceinline__ int4 pack8(const float (&acc)[8], __nv_bfloat16*) {
-  int4 r;
-  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&r);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-  return r;
-}
-
 // ---- phases --------------------------------------------------------------------
 
 template <typename T, bool kLines>
-__device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSmem& sm) {
+__device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSmem& sm, int m) {
   const A2AParams& p = a.p;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
 
-  if (blockIdx.x == 0) {
-    // The dispatch that produced these rows has finished on this rank: clear the
-    // flag set it used and move on to the other one.  No peer can write this set
-    // again before it has seen counts of this rank's next dispatch.
-    const int parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
-    uint32_t* counts = reinterpret_cast<uint32_t*>(p.peer[p.rank] + p.off_counts) +
-                       a2a_counts_index(p, parity, 0, 0);
-    uint32_t* arrived =
-        reinterpret_cast<uint32_t*>(p.peer[p.rank] + p.off_arrived) + parity * p.world;
-    const int P = p.world * p.nle;
-    for (int q = tid; q < P; q += blockDim.x) counts[q] = 0;
-    if (tid < p.world) arrived[tid] = 0;
-    reset_packed_flags(p, parity);
+  if (blockIdx.x == 0) finish_dispatch_round(p);
+  // In a world of one rank the rows are found by (token, k), else by (local expert, row).
+  const bool by_token = p.row_of != nullptr;
+  if (!by_token) {
+    for (int le = tid; le < p.nle; le += blockDim.x) sm.estart[le] = p.recv_count[le];
     __syncthreads();
-    if (tid == 0) {
-      const uint32_t done = *p.iter;
-      // Exactly one dispatch must have started since the last combine.
-      const uint32_t started = ptx::ld_volatile(p.comb_iter);
-      if (started != done + 1u)
-        report_failure(p.status, kOutOfOrder, kPhaseCombinePayload, 0, done + 1u, started, p.rank);
-      *p.iter = done + 1u;
-    }
+    if (warp == 0) warp_exclusive_scan_smem(sm.estart, p.nle, lane, true);
+    __syncthreads();
   }
-  for (int le = tid; le < p.nle; le += blockDim.x) sm.estart[le] = p.recv_count[le];
-  __syncthreads();
-  if (warp == 0) warp_exclusive_scan_smem(sm.estart, p.nle, lane, true);
-  __syncthreads();
   trace(p, kTrCombineLayout);
-  const uint32_t total_rows = sm.estart[p.nle];
+  const uint32_t total_rows =
+      by_token ? static_cast<uint32_t>(m) * static_cast<uint32_t>(p.topk) : sm.estart[p.nle];
+  // {local expert, row} of the f-th row and {source rank | k << 16, token} of its origin.
+  auto find_row = [&](uint32_t f, uint2& place, uint2& rs) {
+    if (by_token) {
+      place = p.row_of[f];
+      rs.y = f / static_cast<uint32_t>(p.topk);
+      rs.x = (f - rs.y * static_cast<uint32_t>(p.topk)) << 16;
+    } else {
+      place.x = static_cast<uint32_t>(find_group(sm.estart, p.nle, f));
+      place.y = f - sm.estart[place.x];
+      rs = p.row_src[static_cast<size_t>(place.x) * p.cap + place.y];
+    }
+  };
 
   const int row_bytes = p.hidden_dim * static_cast<int>(sizeof(T));
   const int nvec = row_bytes >> 4;
@@ -205,9 +140,8 @@ __device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSm
     for (uint32_t unit = gwarp; unit < n_units; unit += gwarps) {
       const uint32_t f = unit / split;
       const int c = static_cast<int>(unit - f * split);
-      const int le = find_group(sm.estart, p.nle, f);
-      const uint32_t row = f - sm.estart[le];
-      const uint2 rs = p.row_src[static_cast<size_t>(le) * p.cap + row];
+      uint2 place, rs;
+      find_row(f, place, rs);
       const int src_rank = static_cast<int>(rs.x & 0xffffu);
       const uint32_t k = rs.x >> 16;
       const uint32_t token = rs.y;
@@ -218,8 +152,9 @@ __device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSm
                          p.rank);
         continue;
       }
+      if (place.x == kNoRow) continue;  // the entry named no expert
       const uint8_t* src = reinterpret_cast<const uint8_t*>(
-          y + le * a.y_stride_e + static_cast<int64_t>(row) * a.y_stride_row);
+          y + place.x * a.y_stride_e + place.y * a.y_stride_row);
       const int l0 = (c * nlines) / split;
       const int l1 = ((c + 1) * nlines) / split;
       const int group_first = (src_rank / p.dp_size) * p.dp_size;
@@ -246,9 +181,8 @@ __device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSm
     if (unit < n_units) {
       const uint32_t f = unit / split;
       const int c = static_cast<int>(unit - f * split);
-      const int le = find_group(sm.estart, p.nle, f);
-      const uint32_t row = f - sm.estart[le];
-      const uint2 rs = p.row_src[static_cast<size_t>(le) * p.cap + row];
+      uint2 place, rs;
+      find_row(f, place, rs);
       const int src_rank = static_cast<int>(rs.x & 0xffffu);
       const uint32_t k = rs.x >> 16;
       const uint32_t token = rs.y;
@@ -257,9 +191,9 @@ __device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSm
         if (lane == 0)
           report_failure(p.status, kBadToken, kPhaseCombinePayload, src_rank, p.max_tokens,
                          token, p.rank);
-      } else {
+      } else if (place.x != kNoRow) {
         const uint8_t* src = reinterpret_cast<const uint8_t*>(
-            y + le * a.y_stride_e + static_cast<int64_t>(row) * a.y_stride_row);
+            y + place.x * a.y_stride_e + place.y * a.y_stride_row);
         const size_t v0 = static_cast<size_t>((c * nvec) / split);
         const int nv = ((c + 1) * nvec) / split - static_cast<int>(v0);
         const int group_first = (src_rank / p.dp_size) * p.dp_size;
@@ -546,7 +480,7 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, uint32_t* sme
   m = min(m, p.max_tokens);
   trace(p, kTrCombineStart);
   trace_block(p, kTrBlockCombineStart);
-  if constexpr (SEND) send_phase<T, kLines>(a, sm);
+  if constexpr (SEND) send_phase<T, kLines>(a, sm, m);
   trace(p, kTrCombineSent);
   if constexpr (SEND && RECV) __syncthreads();
   if constexpr (RECV) {
@@ -606,25 +540,6 @@ cudaError_t launch_typed_multi(const CombineMulti& args, int nranks, bool send, 
                                 : combine_fn<T, U, false, true>(send, recv);
   return cudaLaunchCooperativeKernel(fn, dim3(grid, nranks), dim3(kCombineThreads), params, smem,
                                      stream);
-}
-
-// Calls fn.template operator()<T, U>() for the (in, out) dtype pair.
-template <typename F>
-cudaError_t dispatch_types(DType in, DType out, F&& fn) {
-  const bool out_bf16 = out == DType::kBF16;
-  if (out != DType::kBF16 && out != DType::kF16) return cudaErrorInvalidValue;
-  switch (in) {
-    case DType::kF32:
-      return out_bf16 ? fn.template operator()<float, __nv_bfloat16>()
-                      : fn.template operator()<float, __half>();
-    case DType::kF16:
-      return out_bf16 ? fn.template operator()<__half, __nv_bfloat16>()
-                      : fn.template operator()<__half, __half>();
-    case DType::kBF16:
-      return out_bf16 ? fn.template operator()<__nv_bfloat16, __nv_bfloat16>()
-                      : fn.template operator()<__nv_bfloat16, __half>();
-  }
-  return cudaErrorInvalidValue;
 }
 
 }  // namespace

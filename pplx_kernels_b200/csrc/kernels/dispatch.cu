@@ -57,7 +57,6 @@
 #include <algorithm>
 
 #include <cuda_bf16.h>
-#include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
 #include "../core/device_utils.cuh"
@@ -67,6 +66,7 @@
 #include "../core/wait.cuh"
 #include "a2a_kernels.h"
 #include "a2a_params.h"
+#include "quant_device.cuh"
 
 namespace pplx {
 namespace {
@@ -163,53 +163,15 @@ __device__ __forceinline__ void warp_quantize_row(uint8_t* slot, float* slot_sca
   for (int base = v0; base < v1; base += 32) {
     const int v = base + lane;
     const bool live = v < v1 && v < nvec;
-    float f[16];
-    float amax = 0.f;
+    int4 lo{}, hi{}, q;
+    float scale;
     if (live) {
-      const int4 lo = ptx::ld_nc_v4(src + static_cast<size_t>(v) * 16);
-      const int4 hi = ptx::ld_nc_v4(src + static_cast<size_t>(v) * 16 + 8);
-      const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&lo);
-      const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&hi);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 x = __bfloat1622float2(a[j]);
-        const float2 y = __bfloat1622float2(b[j]);
-        f[2 * j] = x.x;
-        f[2 * j + 1] = x.y;
-        f[8 + 2 * j] = y.x;
-        f[8 + 2 * j + 1] = y.y;
-      }
-#pragma unroll
-      for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
+      lo = ptx::ld_nc_v4(src + static_cast<size_t>(v) * 16);
+      hi = ptx::ld_nc_v4(src + static_cast<size_t>(v) * 16 + 8);
     }
-    // 8 consecutive lanes hold one 128-column block.
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    warp_quantize16(lo, hi, live, pow2, q, scale);
     if (!live) continue;
-    amax = fmaxf(amax, 1e-4f);
-    float scale = amax / 448.0f, inv = 448.0f / amax;
-    if (pow2) {
-      // The smallest power of two that is not below amax / 448: hardware block scaling.
-      const uint32_t bits = __float_as_uint(scale);
-      scale = __uint_as_float(((bits >> 23) + ((bits & 0x7fffffu) != 0u ? 1u : 0u)) << 23);
-      inv = 1.0f / scale;
-    }
-    uint32_t q[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t p0 = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j] * inv, f[4 * j + 1] * inv),
-                                                   __NV_SATFINITE, __NV_E4M3);
-      const uint32_t p1 = __nv_cvt_float2_to_fp8x2(
-          make_float2(f[4 * j + 2] * inv, f[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-      q[j] = p0 | (p1 << 16);
-    }
-    int4 out;
-    out.x = q[0];
-    out.y = q[1];
-    out.z = q[2];
-    out.w = q[3];
-    ptx::st_v4(slot + static_cast<size_t>(v) * 16, out);
+    ptx::st_v4(slot + static_cast<size_t>(v) * 16, q);
     if ((lane & 7) == 0) slot_scales[v >> 3] = scale;
   }
 }

@@ -161,7 +161,11 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
 
   iter_ = DeviceBuffer<uint32_t>(2);
   recv_count_ = DeviceBuffer<uint32_t>(params_.nle);
-  row_src_ = DeviceBuffer<uint2>(static_cast<size_t>(params_.nle) * params_.cap);
+  // (A world of one rank also keeps where each (token, k) went, behind row_src.)
+  const size_t rows = static_cast<size_t>(params_.nle) * params_.cap;
+  const bool single = cfg_.world_size == 1;
+  row_src_ = DeviceBuffer<uint2>(
+      rows + (single ? static_cast<size_t>(params_.max_tokens) * params_.topk : 0));
   status_ = DeviceBuffer<Status>(1);
   status_host_ = HostBuffer<Status>(1, /*mapped=*/true);
   {
@@ -175,6 +179,7 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
   params_.comb_iter = iter_.get() + 1;
   params_.recv_count = recv_count_.get();
   params_.row_src = row_src_.get();
+  params_.row_of = single ? row_src_.get() + rows : nullptr;
   params_.status = status_.get();
   params_.timeout_ns = static_cast<uint64_t>(env_long("PPLX_B200_TIMEOUT_MS", 10000)) * 1000000ull;
   params_.debug_checks = env_long("PPLX_B200_DEBUG_CHECKS", 0) != 0 ? 1 : 0;
@@ -202,9 +207,11 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
     int smem_limit = 0;
     CUDA_CHECK(cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                       current_device()));
-    PPLX_CHECK(dispatch_smem_bytes(params_) <= static_cast<size_t>(smem_limit),
+    const size_t need = single ? std::max(single_rank_smem_bytes(params_), dispatch_smem_bytes(params_))
+                               : dispatch_smem_bytes(params_);
+    PPLX_CHECK(need <= static_cast<size_t>(smem_limit),
                "num_experts " << cfg_.num_experts << " with world_size " << cfg_.world_size
-                              << " needs " << dispatch_smem_bytes(params_)
+                              << " needs " << need
                               << " bytes of shared memory per block for the dispatch histogram; "
                                  "the device offers "
                               << smem_limit);
@@ -329,8 +336,12 @@ void AllToAll::set_timeout_ms(double ms) {
   params_.timeout_ns = static_cast<uint64_t>(ms * 1e6);
 }
 
+int AllToAll::block_limit() const {
+  return max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+}
+
 int AllToAll::dispatch_grid(int num_tokens) const {
-  const int limit = max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+  const int limit = block_limit();
   const int units = std::max(1, num_tokens) * cfg_.experts_per_token;
   return std::clamp(ceil_div(units, 4), std::min(4, limit), limit);
 }
@@ -338,7 +349,7 @@ int AllToAll::dispatch_grid(int num_tokens) const {
 bool AllToAll::dispatch_uses_lines(bool quantize) const { return params_.ll != 0 && !quantize; }
 
 int AllToAll::combine_grid(int num_tokens) const {
-  const int limit = max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+  const int limit = block_limit();
   const int warps = combine_threads() / 32;
   const int chunks = ceil_div(cfg_.hidden_dim / 8, 32);
   const int units = std::max(1, num_tokens) * std::max(cfg_.experts_per_token, chunks);
@@ -440,6 +451,10 @@ void AllToAll::dispatch_send_packed(const DispatchCall& call, cudaStream_t strea
   NvtxRange range("dispatch_send_packed");
   const DispatchArgs a = make_packed_send_args(call);
   begin(Step::kDispatchSend, false);
+  if (cfg_.world_size == 1) {
+    CUDA_CHECK(launch_single_dispatch(a, true, false, block_limit(), stream));
+    return;
+  }
   CUDA_CHECK(launch_dispatch(a, true, false, dispatch_grid(call.num_tokens), stream));
 }
 
@@ -477,6 +492,11 @@ void AllToAll::dispatch_send_packed_group(const std::vector<AllToAll*>& ranks,
                                           cudaStream_t stream) {
   PPLX_CHECK(!ranks.empty() && ranks.size() == calls.size(), "dispatch group: size mismatch");
   check_local_ranks(ranks.size());
+  if (ranks[0]->cfg_.world_size == 1) {
+    PPLX_CHECK(ranks.size() == 1, "a group launch takes ranks of one world");
+    ranks[0]->dispatch_send_packed(calls[0], stream);
+    return;
+  }
   std::vector<DispatchArgs> args;
   int max_tokens = 0;
   for (size_t r = 0; r < ranks.size(); ++r) {
@@ -496,8 +516,12 @@ void AllToAll::dispatch(const DispatchCall& call, SplitMode mode, cudaStream_t s
   const DispatchArgs a = make_dispatch_args(call);
   const bool send = mode != SplitMode::kRecv, recv = mode != SplitMode::kSend;
   begin(send ? Step::kDispatchSend : Step::kDispatchRecv, send && recv);
+  if (cfg_.world_size == 1) {
+    CUDA_CHECK(launch_single_dispatch(a, send, recv, block_limit(), stream));
+    return;
+  }
   if (params_.tiny != 0 && !call.quantize) {
-    const int limit = max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+    const int limit = block_limit();
     CUDA_CHECK(launch_dispatch_tiny(a, send, recv, dispatch_tiny_grid(params_, limit), stream));
     return;
   }
@@ -509,6 +533,11 @@ void AllToAll::combine(const CombineCall& call, SplitMode mode, cudaStream_t str
   CombineArgs a = make_combine_args(call);
   const bool send = mode != SplitMode::kRecv, recv = mode != SplitMode::kSend;
   begin(send ? Step::kCombineSend : Step::kCombineRecv, send && recv);
+  if (cfg_.world_size == 1 && send && recv) {
+    combine_send_used_lines_ = false;
+    CUDA_CHECK(launch_single_combine(a, call.in, call.out, block_limit(), stream));
+    return;
+  }
   // The receive half follows whatever its send half used: lines for a send of this class,
   // counters after the GEMM-epilogue send of the fused MoE path.
   if (send) combine_send_used_lines_ = a.ll != 0;
@@ -534,7 +563,7 @@ void AllToAll::fused_up(const FusedFfnCall& f, cudaStream_t stream) {
   c.k = params_.hidden_dim;
   c.swiglu = true;
   c.expected_total_rows = f.expected_total_rows;
-  c.num_sms = max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+  c.num_sms = block_limit();
   launch_gemm_from_staging(c, params_, f.out_num_tokens, stream);
 }
 
@@ -561,7 +590,7 @@ void AllToAll::fused_up_fp8(const FusedFfnFp8Call& f, cudaStream_t stream) {
   c.k = params_.hidden_dim;
   c.swiglu_quant = true;
   c.pow2_scales = params_.quant_pow2 != 0;
-  c.num_sms = max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+  c.num_sms = block_limit();
   launch_gemm_fp8_from_staging(c, params_, f.out_num_tokens, stream);
 }
 
@@ -590,7 +619,7 @@ void AllToAll::fused_down_fp8(const FusedFfnFp8Call& f, cudaStream_t stream) {
   c.n_out = params_.hidden_dim;
   c.k = f.inter_dim;
   c.swiglu_quant = false;
-  c.num_sms = max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+  c.num_sms = block_limit();
   launch_gemm_fp8_to_peers(c, params_, stream);
 }
 
@@ -613,7 +642,7 @@ void AllToAll::fused_down(const FusedFfnCall& f, cudaStream_t stream) {
   c.k = f.inter_dim;
   c.swiglu = false;
   c.expected_total_rows = f.expected_total_rows;
-  c.num_sms = max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+  c.num_sms = block_limit();
   launch_gemm_to_peers(c, params_, stream);
 }
 
@@ -623,6 +652,11 @@ void AllToAll::dispatch_group(const std::vector<AllToAll*>& ranks,
                               cudaStream_t stream) {
   PPLX_CHECK(!ranks.empty() && ranks.size() == calls.size(), "dispatch_group: size mismatch");
   check_local_ranks(ranks.size());
+  if (ranks[0]->cfg_.world_size == 1) {
+    PPLX_CHECK(ranks.size() == 1, "a group launch takes ranks of one world");
+    ranks[0]->dispatch(calls[0], mode, stream);
+    return;
+  }
   std::vector<DispatchArgs> args;
   int grid = 1, max_tokens = 0;
   for (size_t r = 0; r < ranks.size(); ++r) {
@@ -651,6 +685,11 @@ void AllToAll::combine_group(const std::vector<AllToAll*>& ranks,
                              cudaStream_t stream) {
   PPLX_CHECK(!ranks.empty() && ranks.size() == calls.size(), "combine_group: size mismatch");
   check_local_ranks(ranks.size());
+  if (ranks[0]->cfg_.world_size == 1) {
+    PPLX_CHECK(ranks.size() == 1, "a group launch takes ranks of one world");
+    ranks[0]->combine(calls[0], mode, stream);
+    return;
+  }
   std::vector<CombineArgs> args;
   int max_tokens = 0;
   for (size_t r = 0; r < ranks.size(); ++r) {

@@ -205,6 +205,7 @@ class AllToAll {
 
   DispatchArgs make_dispatch_args(const DispatchCall& call) const;
   CombineArgs make_combine_args(const CombineCall& call) const;
+  int block_limit() const;  // blocks a launch may have at most
   int dispatch_grid(int num_tokens) const;
   int combine_grid(int num_tokens) const;
   // Whether a dispatch of this object moves its rows as flag-in-data lines.
