@@ -63,29 +63,36 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
-// Waits for the phase with the given parity to complete, for at most `limit_ns`.
+// Waits for the phase with the given parity to complete, for at most about `limit_ns`.
 // `abort_flag` is a shared-memory word that any role of the CTA sets when it
 // gives up; once set, every wait returns false at its next check so that the CTA
 // drains to its teardown instead of hanging.
+//
+// The thread sleeps in the barrier unit (a try_wait with a time hint of a millisecond) and is
+// woken by the phase itself; the limit counts those sleeps.  Polling instead, with a look at
+// %globaltimer in between, woke up about a microsecond late and kept the issue slots and the
+// shared-memory port busy that the working warps of the CTA need.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           volatile uint32_t* abort_flag, uint64_t limit_ns) {
-  for (int i = 0; i < 64; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-  }
-  uint64_t t0;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  while (true) {
-    for (int i = 0; i < 16; ++i) {
-      if (mbar_try_wait(bar, parity)) return true;
-    }
+  if (mbar_try_wait(bar, parity)) return true;
+  constexpr uint32_t kSleepNs = 1000000;
+#pragma unroll 1
+  for (uint64_t slept = 0; slept < limit_ns; slept += kSleepNs) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2, %3;\n\t"
+        "selp.b32 %0, 1, 0, P;\n\t"
+        "}\n"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kSleepNs)
+        : "memory");
+    if (done != 0u) return true;
     if (*abort_flag != 0u) return false;
-    uint64_t t1;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-    if (t1 - t0 > limit_ns) {
-      *abort_flag = 1u;
-      return false;
-    }
   }
+  *abort_flag = 1u;
+  return false;
 }
 
 // ----------------------------------------------------------------- TMA ----

@@ -18,6 +18,7 @@ struct Fp8GemmArgs {
   // Only read by the forms fused with the all-to-all:
   int32_t* out_num_tokens;  // optional [nle]: per-expert totals for the caller
   int src_table;            // keep rows per (expert, source) in shared memory
+  uint32_t ring_bytes;      // shared memory for the stages (form with fp32 scales)
   A2AParams a2a;
 };
 
@@ -44,23 +45,24 @@ __device__ __forceinline__ void flush_signals(const A2AParams& p, const Fp8PeerS
 // Staging-fed forms: waits until the rows of tile `c` have landed, that is for the arrival
 // counters of exactly the sources whose rows the tile covers.  `landed` remembers the sources
 // of the current expert that were already waited for.  False: a wait ran out.
-__device__ __forceinline__ bool wait_tile_sources(const A2AParams& p, const Fp8Tile& c, int parity,
-                                                  const uint32_t* src_rows, uint32_t& landed) {
+__device__ __forceinline__ bool wait_tile_sources(const A2AParams& p, int expert, int first_row,
+                                                  int end_row, int parity, const uint32_t* src_rows,
+                                                  uint32_t& landed) {
   const WaitCtx w{p.status, p.timeout_ns, static_cast<uint32_t>(p.rank)};
   const uint32_t* arrived = reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_arrived_e) +
-                            (static_cast<size_t>(parity) * p.nle + c.expert) * p.world;
-  const uint32_t r0 = static_cast<uint32_t>(c.m_blk * kBlockM);
-  const uint32_t r1 = min(r0 + static_cast<uint32_t>(kBlockM), static_cast<uint32_t>(c.rows));
+                            (static_cast<size_t>(parity) * p.nle + expert) * p.world;
+  const uint32_t r0 = static_cast<uint32_t>(first_row);
+  const uint32_t r1 = static_cast<uint32_t>(end_row);
   uint32_t first = 0;
   bool waited = false, ok = true;
   for (int s = 0; s < p.world && ok; ++s) {
     uint32_t n;
     if (src_rows != nullptr) {
-      n = src_rows[c.expert * p.world + s];
+      n = src_rows[expert * p.world + s];
     } else {
       const uint32_t v = ptx::ld_relaxed_sys(
           reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_counts_all) +
-          (static_cast<size_t>(parity) * p.world + s) * p.num_experts + p.rank * p.nle + c.expert);
+          (static_cast<size_t>(parity) * p.world + s) * p.num_experts + p.rank * p.nle + expert);
       n = v > 1u ? v - 1u : 0u;
     }
     if (n > 0 && first < r1 && first + n > r0 && !((landed >> s) & 1u)) {
@@ -212,7 +214,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             last_group = c.expert;
             landed = 0;
           }
-          ok = wait_tile_sources(p, c, parity, src_rows, landed);
+          ok = wait_tile_sources(p, c.expert, c.m_blk * kBlockM, min((c.m_blk + 1) * kBlockM, c.rows), parity,
+                                 src_rows, landed);
           if (!ok) {
             *abort_flag = 1u;
             break;
@@ -340,7 +343,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           sf_landed = 0;
         }
         int good = 1;
-        if (lane == 0) good = wait_tile_sources(p, c, parity, src_rows, sf_landed) ? 1 : 0;
+        if (lane == 0) good = wait_tile_sources(p, c.expert, c.m_blk * kBlockM,
+                                             min((c.m_blk + 1) * kBlockM, c.rows), parity, src_rows,
+                                             sf_landed) ? 1 : 0;
         good = __shfl_sync(0xffffffffu, good, 0);
         __syncwarp();
         if (good == 0) {

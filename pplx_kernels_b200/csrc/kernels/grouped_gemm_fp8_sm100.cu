@@ -130,6 +130,7 @@ __device__ __forceinline__ Fp8Tile locate(const uint32_t* tile_start, const uint
 }  // namespace pplx
 
 #include "grouped_gemm_fp8_kernel.inl"
+#include "grouped_gemm_fp8_fold.inl"
 
 namespace pplx {
 namespace {
@@ -154,7 +155,7 @@ EncodeTiledFn encode_tiled_fp8() {
 // [experts, rows, k] one-byte elements with k contiguous; tiles of 128 B x 128 rows x 1,
 // 128-byte swizzle, out-of-range elements read as zero.
 CUtensorMap make_byte_map(const void* base, int64_t experts, int64_t rows, int64_t k,
-                          int64_t stride_row, int64_t stride_expert) {
+                          int64_t stride_row, int64_t stride_expert, int box_rows = 128) {
   PPLX_CHECK(reinterpret_cast<uintptr_t>(base) % 16 == 0 && stride_row % 16 == 0 &&
                  stride_expert % 16 == 0,
              "fp8 operands must be 16-byte aligned with strides that are multiples of 16");
@@ -163,7 +164,7 @@ CUtensorMap make_byte_map(const void* base, int64_t experts, int64_t rows, int64
                               static_cast<cuuint64_t>(experts)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(stride_row),
                                  static_cast<cuuint64_t>(stride_expert)};
-  const cuuint32_t box[3] = {kBlockKBytes, 128, 1};
+  const cuuint32_t box[3] = {kBlockKBytes, static_cast<cuuint32_t>(box_rows), 1};
   const cuuint32_t elem_strides[3] = {1, 1, 1};
   const CUresult r = encode_tiled_fp8()(
       &map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box,
@@ -237,6 +238,37 @@ void launch_fp8(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b, const Fp8G
   CUDA_CHECK(cudaGetLastError());
 }
 
+// Token rows come in boxes of 64 and 16.
+struct TokenMaps {
+  CUtensorMap x64, x16;
+};
+
+TokenMaps make_token_maps(const void* base, int64_t planes, int64_t rows, int64_t k,
+                          int64_t stride_row, int64_t stride_plane) {
+  return {make_byte_map(base, planes, rows, k, stride_row, stride_plane, 64),
+          make_byte_map(base, planes, rows, k, stride_row, stride_plane, 16)};
+}
+
+template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers>
+void launch_fold(const CUtensorMap& tmap_w, const TokenMaps& x, Fp8GemmArgs g, int num_sms,
+                 cudaStream_t stream) {
+  auto* kernel = fold::grouped_gemm_fp8_fold_kernel<kSwiGLUQuant, kFromStaging, kToPeers>;
+  const size_t src_entries =
+      (kFromStaging && g.src_table != 0) ? static_cast<size_t>(g.num_experts) * g.a2a.world : 0;
+  const size_t fixed = 1024 + sizeof(fold::Control) + (kToPeers ? sizeof(fold::PeerStage) : 0) +
+                       sizeof(uint32_t) * (3 * static_cast<size_t>(g.num_experts) + 1 + src_entries);
+  // The stages take what the tables leave: four of the widest tiles fit beside any table the
+  // checks admit.
+  constexpr size_t kSmem = 227 * 1024;
+  g.ring_bytes = static_cast<uint32_t>((kSmem - fixed) & ~static_cast<size_t>(1023));
+  const size_t smem = fixed + g.ring_bytes;
+  CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)));
+  const int grid = num_sms > 0 ? num_sms : get_sm_count();
+  kernel<<<grid, kThreads, smem, stream>>>(tmap_w, x.x64, x.x16, g);
+  CUDA_CHECK(cudaGetLastError());
+}
+
 }  // namespace
 
 void launch_grouped_gemm_fp8(const Fp8GemmCall& c, cudaStream_t stream) {
@@ -250,11 +282,12 @@ void launch_grouped_gemm_fp8(const Fp8GemmCall& c, cudaStream_t stream) {
   if (c.pow2_scales) {
     if (c.swiglu_quant) launch_fp8<true, false, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
     else launch_fp8<false, false, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
-  } else if (c.swiglu_quant) {
-    launch_fp8<true, false, false>(tmap_a, tmap_b, g, c.num_sms, stream);
-  } else {
-    launch_fp8<false, false, false>(tmap_a, tmap_b, g, c.num_sms, stream);
+    return;
   }
+  const TokenMaps x = make_token_maps(c.x, c.num_experts, c.rows_per_expert, c.k, c.x_stride_row,
+                                      c.x_stride_e);
+  if (c.swiglu_quant) launch_fold<true, false, false>(tmap_b, x, g, c.num_sms, stream);
+  else launch_fold<false, false, false>(tmap_b, x, g, c.num_sms, stream);
 }
 
 void launch_gemm_fp8_from_staging(const Fp8GemmCall& c, const A2AParams& p,
@@ -276,8 +309,13 @@ void launch_gemm_fp8_from_staging(const Fp8GemmCall& c, const A2AParams& p,
   g.out_num_tokens = out_num_tokens;
   g.a2a = p;
   g.src_table = static_cast<size_t>(p.nle) * p.world <= kMaxSrcEntriesFp8 ? 1 : 0;
-  if (c.pow2_scales) launch_fp8<true, true, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
-  else launch_fp8<true, true, false>(tmap_a, tmap_b, g, c.num_sms, stream);
+  if (c.pow2_scales) {
+    launch_fp8<true, true, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
+    return;
+  }
+  const TokenMaps x = make_token_maps(p.peer[p.rank] + p.off_disp_stage, 1, slots, p.hidden_dim,
+                                      p.slot_bytes, slots * p.slot_bytes);
+  launch_fold<true, true, false>(tmap_b, x, g, c.num_sms, stream);
 }
 
 void launch_gemm_fp8_to_peers(const Fp8GemmCall& c, const A2AParams& p, cudaStream_t stream) {
@@ -295,8 +333,13 @@ void launch_gemm_fp8_to_peers(const Fp8GemmCall& c, const A2AParams& p, cudaStre
   Fp8GemmArgs g = fp8_args(c);
   g.out = nullptr;
   g.a2a = p;
-  if (c.pow2_scales) launch_fp8<false, false, true, true>(tmap_a, tmap_b, g, c.num_sms, stream);
-  else launch_fp8<false, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
+  if (c.pow2_scales) {
+    launch_fp8<false, false, true, true>(tmap_a, tmap_b, g, c.num_sms, stream);
+    return;
+  }
+  const TokenMaps x = make_token_maps(c.x, c.num_experts, c.rows_per_expert, c.k, c.x_stride_row,
+                                      c.x_stride_e);
+  launch_fold<false, false, true>(tmap_b, x, g, c.num_sms, stream);
 }
 
 }  // namespace pplx
