@@ -132,6 +132,31 @@ __device__ __forceinline__ void tma_load_3d_2cta(void* smem_dst, const void* tma
       : "memory");
 }
 
+// The same two for a tensor map of five dimensions.
+__device__ __forceinline__ void tma_load_5d(void* smem_dst, const void* tmap, uint64_t* bar,
+                                            int crd0, int crd1, int crd2, int crd3, int crd4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)),
+        "r"(crd0), "r"(crd1), "r"(crd2), "r"(crd3), "r"(crd4)
+      : "memory");
+}
+
+__device__ __forceinline__ void tma_load_5d_2cta(void* smem_dst, const void* tmap,
+                                                 uint64_t* leader_bar, int crd0, int crd1, int crd2,
+                                                 int crd3, int crd4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)),
+        "r"(smem_u32(leader_bar) & kPeerBitMask), "r"(crd0), "r"(crd1), "r"(crd2), "r"(crd3),
+        "r"(crd4)
+      : "memory");
+}
+
 // ------------------------------------------------------------- clusters ----
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {

@@ -11,8 +11,6 @@
 
 namespace pplx {
 
-constexpr int kNumTileWidths = 5;
-
 // Device-side arguments (the tensor maps travel as separate kernel parameters).
 struct GroupedGemmArgs {
   const int32_t* counts;   // [num_experts] valid rows per expert
@@ -24,8 +22,8 @@ struct GroupedGemmArgs {
   int rows_per_expert;     // capacity of x / out per expert
   int n_out;               // output columns (the intermediate size for SwiGLU)
   int k;
-  int widths[kNumTileWidths];  // candidate weight rows per B half (the tile is twice as wide
-                               // in columns); 0 = not available.  Chosen on the device.
+  int max_tokens;          // most token rows per tile; the device may choose fewer
+  uint32_t ring_bytes;     // shared memory of the stages (set by the launcher)
   // Only read by the kernels fused with the all-to-all:
   int32_t* out_num_tokens;          // optional [nle]: per-expert totals for the caller
   int src_table;                    // staging-fed form: keep rows per (expert, source) in
@@ -53,10 +51,11 @@ struct GroupedGemmCall {
   int k = 0;
   bool swiglu = false;
   int num_sms = 0;           // 0 = all
-  int half_n = 0;            // 0 = choose; else weight rows per B half (multiple of 8, 64..128)
-  int64_t expected_total_rows = 0;  // hint for the tile-width choice; 0 = capacity
-  int cta_pair = -1;         // -1 = choose, 0 = one CTA per 128-row tile, 1 = CTA pair per
-                             // 256-row tile (tcgen05 cta_group::2)
+  int half_n = 0;            // 0 = choose; else half of the most token rows per tile, which are
+                             // the accumulator's columns (multiple of 8, 16..128)
+  int64_t expected_total_rows = 0;  // kept for callers; the device reads the real counts
+  int cta_pair = -1;         // 0 = one CTA per tile of 128 weight rows, else a CTA pair per
+                             // 256 weight rows (tcgen05 cta_group::2) where the grid has two CTAs
 };
 
 // out[e, :counts[e]] = act(x[e, :counts[e]] @ w[e]^T); rows beyond counts[e] are untouched.

@@ -37,8 +37,9 @@ namespace pplx {
 namespace {
 namespace fold {
 
+using namespace tok;
+
 constexpr int kMaxStages = 12;
-constexpr int kQueue = 512;          // kToPeers: arrival adds that wait for one fence
 constexpr int kSegBytes = 256 + 16;  // 128 columns of bf16 of one token, padded
 constexpr int kBuffers = 4;          // scratch accumulators of 128 columns of tensor memory
 
@@ -72,20 +73,6 @@ struct Control {
   alignas(16) uint8_t seg[2][2][16][kSegBytes];  // [warp group][alternating][token][column]
 };
 
-struct PeerStage {
-  unsigned long long row_off[256];      // arena offset of each token's combine slot
-  uint32_t token[256];                  // kNoSignalFp8: none
-  uint32_t group[256];                  // first rank of the token's DP group
-  uint32_t q_token[kQueue];
-  uint32_t q_group_units[kQueue];
-};
-
-// Token tile of an expert: the fewest tiles of at most `most`, all of one width.
-__device__ __forceinline__ int token_tiles(int rows, int most) { return (rows + most - 1) / most; }
-__device__ __forceinline__ int token_width(int rows, int tiles) {
-  return (((rows + tiles - 1) / tiles) + 15) & ~15;
-}
-
 // Tiles of an expert are ordered with the token tile fastest: CTAs that run at the same time
 // share a block of weights in L2.
 template <int kHalves>
@@ -116,26 +103,11 @@ __device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// 16 lanes x 16 columns: thread t receives columns 2 * (t % 4) and the next one of lane t / 4
-// (r[0], r[1]) and of lane t / 4 + 8 (r[2], r[3]), then the same of the next eight columns.
-__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7])
-      : "r"(taddr));
-}
-
 // A group of 16 tokens times this warp's 32 weight rows, as a thread holds it: pair[2 * q + b] is
 // tokens {8 * b + 2 * (t % 4), + 1} of row 8 * q + t / 4.
 struct Group {
   uint64_t pair[8];
 };
-
-__device__ __forceinline__ void load_group(uint32_t taddr, uint32_t (&lo)[8], uint32_t (&hi)[8]) {
-  tmem_ld_16x256b_x2(taddr, lo);
-  tmem_ld_16x256b_x2(taddr + (16u << 16), hi);
-}
 
 // acc += part * scale; `scales` points at the group's 16 products.
 __device__ __forceinline__ void fold_group(Group& acc, const uint32_t (&lo)[8],
@@ -150,24 +122,10 @@ __device__ __forceinline__ void fold_group(Group& acc, const uint32_t (&lo)[8],
   }
 }
 
-// Stores four 8 x 8 blocks of 16-bit values (32 weight rows x 8 tokens) with the token as row:
-// lane l gives the address of token l % 8 of block l / 8.
-__device__ __forceinline__ void stmatrix_x4_trans(void* smem, uint32_t r0, uint32_t r1, uint32_t r2,
-                                                  uint32_t r3) {
-  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(
-                   tc::smem_u32(smem)),
-               "r"(r0), "r"(r1), "r"(r2), "r"(r3)
-               : "memory");
-}
-
 __device__ __forceinline__ uint32_t bf16_pair(uint64_t v) {
   const float2 f = unpack2(v);
   const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
   return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-__device__ __forceinline__ void sync_group(int wg) {
-  asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory");
 }
 
 struct FoldLoop {
@@ -239,21 +197,6 @@ __device__ __forceinline__ bool fold_tile(const FoldLoop& f, int own,
     if (own < kOwn) return fold_tile<kHalves, kOwn - 1>(f, own, acc, round);
   }
   return fold_k_loop<kHalves, kOwn>(f, acc, round);
-}
-
-// One fence, then the queued adds on the tokens' arrival counters (one warp).
-__device__ __forceinline__ void flush(const A2AParams& p, const PeerStage* st, uint32_t count,
-                                      int lane) {
-  ptx::fence_acq_rel_sys();
-  for (uint32_t i = lane; i < count; i += 32) {
-    const uint32_t grp = st->q_group_units[i] & 0xffu;
-    const uint32_t units = st->q_group_units[i] >> 8;
-    for (int r = 0; r < min(p.dp_size, 8); ++r) {
-      ptx::red_add_relaxed_sys(
-          reinterpret_cast<uint32_t*>(p.peer[grp + r] + p.off_comb_arrived) + st->q_token[i], units);
-    }
-  }
-  __syncwarp();
 }
 
 template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers>
@@ -618,7 +561,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // Where each token's row goes, and whose token it is.
         if (n_tid < c.width) {
           unsigned long long off = 0;
-          uint32_t sig_token = kNoSignalFp8, sig_group = 0;
+          uint32_t sig_token = kNoSignal, sig_group = 0;
           if (n_tid < live) {
             const uint2 rs = p.row_src[static_cast<size_t>(c.expert) * p.cap + c.first + n_tid];
             const int src_rank = static_cast<int>(rs.x & 0xffffu);
@@ -728,7 +671,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int4 v = *reinterpret_cast<const int4*>(&seg[tok][(lt & 15) * 16]);
             if (col + 8 > g.n_out) continue;
             if constexpr (kToPeers) {
-              if (peer_stage->token[n] != kNoSignalFp8) {
+              if (peer_stage->token[n] != kNoSignal) {
                 const uint32_t first_rank = peer_stage->group[n];
                 const size_t off = peer_stage->row_off[n] + static_cast<size_t>(col) * 2;
                 for (int r = 0; r < min(p.dp_size, 8); ++r) ptx::st_v4(p.peer[first_rank + r] + off, v);
@@ -753,8 +696,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             pending_signals = 0;
           }
           for (int j0 = 0; j0 < c.width; j0 += 32) {
-            const uint32_t tok = j0 + lane < c.width ? peer_stage->token[j0 + lane] : kNoSignalFp8;
-            const bool there = tok != kNoSignalFp8;
+            const uint32_t tok = j0 + lane < c.width ? peer_stage->token[j0 + lane] : kNoSignal;
+            const bool there = tok != kNoSignal;
             const uint32_t mask = __ballot_sync(0xffffffffu, there);
             if (there) {
               const uint32_t at = pending_signals + __popc(mask & ((1u << lane) - 1u));

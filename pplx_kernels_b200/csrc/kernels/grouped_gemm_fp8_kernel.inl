@@ -41,42 +41,6 @@ __device__ __forceinline__ void flush_signals(const A2AParams& p, const Fp8PeerS
 // kFromStaging: the A operand and its scales are read out of the dispatch staging arena
 // that peers fill (packed, quantising send); tiles wait for the sources they cover.
 // kToPeers: the bf16 result rows go to the combine staging of the tokens' home ranks.
-// Same protocol as the bf16 kernel's forms of the same names (grouped_gemm_sm100.cu).
-// Staging-fed forms: waits until the rows of tile `c` have landed, that is for the arrival
-// counters of exactly the sources whose rows the tile covers.  `landed` remembers the sources
-// of the current expert that were already waited for.  False: a wait ran out.
-__device__ __forceinline__ bool wait_tile_sources(const A2AParams& p, int expert, int first_row,
-                                                  int end_row, int parity, const uint32_t* src_rows,
-                                                  uint32_t& landed) {
-  const WaitCtx w{p.status, p.timeout_ns, static_cast<uint32_t>(p.rank)};
-  const uint32_t* arrived = reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_arrived_e) +
-                            (static_cast<size_t>(parity) * p.nle + expert) * p.world;
-  const uint32_t r0 = static_cast<uint32_t>(first_row);
-  const uint32_t r1 = static_cast<uint32_t>(end_row);
-  uint32_t first = 0;
-  bool waited = false, ok = true;
-  for (int s = 0; s < p.world && ok; ++s) {
-    uint32_t n;
-    if (src_rows != nullptr) {
-      n = src_rows[expert * p.world + s];
-    } else {
-      const uint32_t v = ptx::ld_relaxed_sys(
-          reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_counts_all) +
-          (static_cast<size_t>(parity) * p.world + s) * p.num_experts + p.rank * p.nle + expert);
-      n = v > 1u ? v - 1u : 0u;
-    }
-    if (n > 0 && first < r1 && first + n > r0 && !((landed >> s) & 1u)) {
-      uint32_t seen;
-      ok = wait_until(arrived + s, PredGe{n}, seen, w, kPhaseFusedGemm, static_cast<uint32_t>(s), n);
-      landed |= 1u << s;
-      waited = true;
-    }
-    first += n;
-  }
-  if (ok && waited) ptx::fence_proxy_async();
-  return ok;
-}
-
 // E8M0 byte of a power-of-two fp32 scale (its exponent field).
 __device__ __forceinline__ uint32_t e8m0_of(float scale) {
   return (__float_as_uint(scale) >> 23) & 0xffu;
@@ -214,7 +178,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             last_group = c.expert;
             landed = 0;
           }
-          ok = wait_tile_sources(p, c.expert, c.m_blk * kBlockM, min((c.m_blk + 1) * kBlockM, c.rows), parity,
+          ok = tok::wait_tile_sources(p, c.expert, c.m_blk * kBlockM, min((c.m_blk + 1) * kBlockM, c.rows), parity,
                                  src_rows, landed);
           if (!ok) {
             *abort_flag = 1u;
@@ -343,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           sf_landed = 0;
         }
         int good = 1;
-        if (lane == 0) good = wait_tile_sources(p, c.expert, c.m_blk * kBlockM,
+        if (lane == 0) good = tok::wait_tile_sources(p, c.expert, c.m_blk * kBlockM,
                                              min((c.m_blk + 1) * kBlockM, c.rows), parity, src_rows,
                                              sf_landed) ? 1 : 0;
         good = __shfl_sync(0xffffffffu, good, 0);

@@ -47,6 +47,7 @@
 #include "../core/wait.cuh"
 #include "a2a_device.cuh"
 #include "grouped_gemm.h"
+#include "token_tile.cuh"
 
 namespace pplx {
 namespace {
@@ -255,7 +256,7 @@ void launch_fold(const CUtensorMap& tmap_w, const TokenMaps& x, Fp8GemmArgs g, i
   auto* kernel = fold::grouped_gemm_fp8_fold_kernel<kSwiGLUQuant, kFromStaging, kToPeers>;
   const size_t src_entries =
       (kFromStaging && g.src_table != 0) ? static_cast<size_t>(g.num_experts) * g.a2a.world : 0;
-  const size_t fixed = 1024 + sizeof(fold::Control) + (kToPeers ? sizeof(fold::PeerStage) : 0) +
+  const size_t fixed = 1024 + sizeof(fold::Control) + (kToPeers ? sizeof(tok::PeerStage) : 0) +
                        sizeof(uint32_t) * (3 * static_cast<size_t>(g.num_experts) + 1 + src_entries);
   // The stages take what the tables leave: four of the widest tiles fit beside any table the
   // checks admit.

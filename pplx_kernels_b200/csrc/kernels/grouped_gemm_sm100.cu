@@ -5,36 +5,40 @@
 // ([2 * I, K]) and the result has I columns: silu(x @ gate^T) * (x @ up^T).
 //
 // The reference contains no GEMM; this kernel serves the fused MoE layer that
-// goes beyond it.  Design (one CTA per SM, persistent over tiles):
+// goes beyond it.
 //
-//   warp 0      TMA producer: cp.async.bulk.tensor tile loads of x and w into a
-//               ring of 128-byte-swizzled shared-memory stages (no multicast)
-//   warp 1      one elected thread issues tcgen05.mma (M=128, N=256, K=16 per
-//               instruction) into one of two 256-column accumulators in tensor
-//               memory, and tcgen05.commit to hand stages and accumulators on
-//   warp 2      allocates / frees the 512 tensor-memory columns
-//   warps 4-7   epilogue: tcgen05.ld of the finished accumulator, activation,
-//               bf16 conversion, masked 16-byte global stores; overlaps with the
-//               MMAs of the next tile through the second accumulator
+// The WEIGHTS are the M operand of the MMAs and the tokens the N operand.  A CTA pair
+// (tcgen05 cta_group::2) owns a tile of 256 weight rows, 128 in each CTA's tensor-memory
+// lanes, times a token tile of 32 to 256 rows of one expert in steps of 32; each CTA loads its
+// own weight rows and HALF of the tokens, and the leader's MMAs read both CTAs' shared
+// memory.  An expert's rows are cut into equal token tiles (to a step), so
+//   - weights cross from DRAM once and from L2 once for up to 256 rows of an expert,
+//   - the work follows the rows there are, to a multiple of 32: with the tokens as M every
+//     expert was padded to a multiple of 128 rows (256 for pairs, which therefore were only
+//     used from 2048 rows per expert on),
+//   - a pair reads 64 bytes per SM and clock from L2 at the full MMA rate; one CTA per
+//     128 x 256 tile needs 96, and L2 delivers about 64: that bound the kernel at 1.0 PFLOP/s.
+// The SwiGLU form interleaves eight gate rows with eight up rows in shared memory (a
+// five-dimensional tensor map does that on the way), so that the 16x256b reads of tensor memory
+// give a thread both halves of its results.
 //
-// With kTwoCta the kernel runs as clusters of two CTAs that share one 256-row tile
-// (tcgen05 cta_group::2): each CTA loads its own 128 rows of A and HALF of the
-// weight tile, the leader CTA issues M = 256 MMAs that read both CTAs' shared
-// memory, and each CTA keeps and drains the accumulator of its own 128 rows.
-// Per SM that halves the weight traffic into shared memory and the shared-memory
-// reads per MMA, which is what limits the one-CTA form.  No TMA multicast is
-// involved: the two CTAs load different data; only barrier arrivals
-// (tcgen05.commit) are delivered to both CTAs.
+// Layers before and after: Mixtral 8x7B (8 experts of 14336 x 4096) with 512 tokens 647 -> 543 us
+// and with 4096 tokens 2867 -> 2640 us, Qwen3-30B-A3B (128 experts of 768 x 2048) with 16 tokens
+// 191 -> 158 us.
 //
-// Tiles are (expert, 256-column block, 128-row block) with the row block varying
-// fastest, so CTAs that run at the same time share a weight tile in L2.  The
-// row counts are read on the device, so the launch is graph-capturable and does
-// no work for empty experts.
+// Roles (persistent over tiles): warp 0 TMA producer, warp 1 MMA issuer (leader CTA only),
+// warp 2 tensor-memory allocation, warps 4-11 epilogue.  Two accumulators of 256 columns let
+// the epilogue of a tile run under the MMAs of the next.  No TMA multicast is involved: the two
+// CTAs load different data; only barrier arrivals (tcgen05.commit) are delivered to both.
+//
+// Tiles are (expert, block of weight rows, token tile) with the token tile varying fastest, so
+// CTAs that run at the same time share weights in L2.  The row counts are read on the device,
+// so the launch is graph-capturable and does no work for empty experts.
 //
 // Two template switches turn the same pipeline into the compute+collective
 // kernels of the fused MoE layer:
 //
-//   kFromStaging   the A operand is read by TMA straight out of the dispatch
+//   kFromStaging   the tokens are read by TMA straight out of the dispatch
 //                  staging arena that PEERS fill with P2P stores (packed send:
 //                  rows grouped by local expert, then by source rank, dense).
 //                  Arrival is counted per (expert, source): before a tile the
@@ -45,9 +49,9 @@
 //                  (source, token, k) of every row for combine.
 //   kToPeers       the epilogue does not write a local result: every output row
 //                  is stored into the combine staging of the token's home rank(s)
-//                  over NVLink, followed once per tile by one system-scope fence
-//                  and relaxed adds on the tokens' arrival counters.  The
-//                  combine send kernel and the expert_y round trip disappear.
+//                  over NVLink in 256-byte pieces, followed by a system-scope fence
+//                  per handful of tiles and relaxed adds on the tokens' arrival counters.
+//                  The combine send kernel and the expert_y round trip disappear.
 //
 // Every mbarrier wait is bounded: when one runs out the CTA raises a shared
 // abort flag, all roles leave their loops, in-flight TMA loads are drained,
@@ -65,96 +69,75 @@
 #include "../core/wait.cuh"
 #include "a2a_device.cuh"
 #include "grouped_gemm.h"
+#include "token_tile.cuh"
 
 namespace pplx {
 namespace {
 
-constexpr int kBlockM = 128;
-constexpr int kBlockN = 256;
-constexpr int kBlockK = 64;   // 64 bf16 = one 128-byte swizzle row
+using namespace tok;
+
+constexpr int kBlockM = 128;      // weight rows per CTA and tile
+constexpr int kMaxTokens = 256;   // token rows per tile
+constexpr int kBlockK = 64;       // 64 bf16 = one 128-byte swizzle row
 constexpr int kUmmaK = 16;
-constexpr int kStages = 4;      // one CTA per tile: 16 KiB of A + 32 KiB of B per stage
-constexpr int kStages2 = 6;     // CTA pair: 16 KiB of A + 16 KiB of B per stage and CTA
-constexpr int kMaxStages = 6;
-constexpr int kThreads = 256;
-constexpr int kTmemCols = 512;
-constexpr uint32_t kABytes = kBlockM * kBlockK * 2;  // 16 KiB
-constexpr uint32_t kBBytes = kBlockN * kBlockK * 2;  // 32 KiB
-constexpr uint32_t kStageBytes = kABytes + kBBytes;
-constexpr uint32_t kStageBytes2 = kABytes + kBBytes / 2;
-constexpr uint64_t kWaitLimitNs = 2000000000ull;     // 2 s per wait
+constexpr int kMaxStages = 12;
+constexpr int kThreads = 384;
+constexpr int kTmemCols = 512;    // two accumulators of kMaxTokens columns
+constexpr uint32_t kRowBytes = kBlockK * 2;
+constexpr uint32_t kWBytes = kBlockM * kRowBytes;
+constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s per wait
 constexpr int kMaxExperts = 1024;
+constexpr int kTileOverhead = 16;     // ... of a tile, in token rows
+constexpr int kSegBytes = 256 + 16;  // 128 bf16 columns of one token, padded
 
-constexpr uint32_t kNoSignal = 0xffffffffu;
-
-// Peer-storing epilogue: an epilogue thread owns one ROW of the tile, so storing straight from
-// registers would send 32 separate 16-byte pieces per instruction over NVLink.  Each epilogue
-// warp therefore passes 64 columns at a time through a [32 rows][128 B + 16 B pad] buffer in
-// shared memory and writes them out as 128-byte row segments (eight lanes per row).
-constexpr int kOutStageRowBytes = 144;
-struct PeerStage {
-  uint8_t rows[4][32][kOutStageRowBytes];   // one buffer per epilogue warp
-  unsigned long long row_off[2][kBlockM];   // arena offset of each tile row's combine slot
-};
-
-// One tensor map of the weights per candidate tile width (the TMA box height is
-// fixed in the map); the kernel picks the width once it knows the real row counts.
-struct WeightMaps {
-  CUtensorMap m[kNumTileWidths];
-};
-
-struct SharedControl {
+struct Control {
   uint64_t full[kMaxStages];
   uint64_t empty[kMaxStages];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   uint32_t abort_flag;
-  uint32_t pad[2];
-  uint32_t sig_token[2][kBlockM];  // kToPeers: token of each tile row, per accumulator
-  uint32_t sig_group[2][kBlockM];  //           first rank of the token's DP group
+  uint32_t max_rows;                // rows of the largest expert
+  uint32_t max_width;               // widest token tile of this launch
+  unsigned long long best_limit;    // (cost << 16) | limit of the token tile
+  alignas(16) uint8_t seg[2][2][16][kSegBytes];  // [warp group][alternating][token][column]
 };
 
-// Rows of A that share a weight matrix: one group per local expert.  With
-// kFromStaging the rows of all experts sit back to back in one plane of A and
-// a_row0 is the expert's first row there.
-struct GroupTable {
-  uint32_t* tile_start;  // [G + 1] first tile of each group
-  uint32_t* rows;        // [G] valid rows
-  uint32_t* a_row0;      // [G] first row inside the A plane
-  uint32_t* out_row0;    // [G] first row inside the output plane
-  uint32_t* src_rows;    // kFromStaging: [G][world] rows that each source sends to the group,
-                         // or null when the table does not fit (then a tile waits for all
-                         // sources of its expert)
+// Token rows come in boxes of 64 and 16.
+struct TokenMaps {
+  CUtensorMap x64, x16;
 };
 
-struct TileCoord {
-  int group;
-  int m_blk;
-  int n_blk;
-  int rows;      // valid rows of the group
-  int a_plane;   // dim-2 coordinate of A
-  int a_row0;
-  int w_plane;   // expert whose weights apply
-  int out_row0;
+struct Tile {
+  int expert;
+  int w_blk;    // block of weight rows (of the pair or the single CTA)
+  int first;    // first token row of the tile inside its expert
+  int width;    // token rows of the tile, a multiple of kUnit
+  int rows;     // valid rows of the expert
 };
 
-// Tiles of one group are ordered (n_blk, m_blk) with m_blk fastest.
-template <bool kFromStaging>
-__device__ __forceinline__ TileCoord locate_tile(const GroupTable& gt, int num_groups,
-                                                 const A2AParams& p, uint32_t t, int tile_m) {
-  TileCoord c;
-  c.group = find_group(gt.tile_start, num_groups, t);
-  c.rows = static_cast<int>(gt.rows[c.group]);
-  const int m_tiles = ceil_div<int>(c.rows, tile_m);
-  const uint32_t rem = t - gt.tile_start[c.group];
-  c.n_blk = static_cast<int>(rem / m_tiles);
-  c.m_blk = static_cast<int>(rem - static_cast<uint32_t>(c.n_blk) * m_tiles);
-  c.a_row0 = static_cast<int>(gt.a_row0[c.group]);
-  c.out_row0 = static_cast<int>(gt.out_row0[c.group]);
-  c.w_plane = c.group;
-  c.a_plane = kFromStaging ? 0 : c.group;
-  (void)p;
+// Token tiles of an expert: as few as `limit` rows per tile allow, as equal as whole units allow.
+template <int kUnit>
+struct Cut {
+  int units, tiles;
+  __device__ __forceinline__ Cut(int rows, int limit)
+      : units((rows + kUnit - 1) / kUnit), tiles((units * kUnit + limit - 1) / limit) {}
+  __device__ __forceinline__ int widest() const { return (units + tiles - 1) / tiles * kUnit; }
+};
+
+template <int kUnit>
+__device__ __forceinline__ Tile locate(const uint32_t* tile_start, const uint32_t* rows_of,
+                                       int num_experts, int limit, uint32_t t) {
+  Tile c;
+  c.expert = find_group(tile_start, num_experts, t);
+  c.rows = static_cast<int>(rows_of[c.expert]);
+  const Cut<kUnit> cut(c.rows, limit);
+  const uint32_t rem = t - tile_start[c.expert];
+  c.w_blk = static_cast<int>(rem / cut.tiles);
+  const int i = static_cast<int>(rem) - c.w_blk * cut.tiles;
+  const int each = cut.units / cut.tiles, wider = cut.units - each * cut.tiles;
+  c.width = (each + (i < wider ? 1 : 0)) * kUnit;
+  c.first = (i * each + min(i, wider)) * kUnit;
   return c;
 }
 
@@ -165,51 +148,89 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kTwoCta>
+__device__ __forceinline__ uint32_t pack_bits(uint32_t a, uint32_t b) {
+  return pack_bf16(__uint_as_float(a), __uint_as_float(b));
+}
+
+// Two tokens' results of one column from their gate and up sums.
+__device__ __forceinline__ uint32_t swiglu_pair(uint32_t g0, uint32_t g1, uint32_t u0, uint32_t u1) {
+  return pack_bf16(silu(__uint_as_float(g0)) * __uint_as_float(u0),
+                   silu(__uint_as_float(g1)) * __uint_as_float(u1));
+}
+
+template <bool kPair>
+__device__ __forceinline__ void load_rows(void* dst, const CUtensorMap* map, uint64_t* full, int k,
+                                          int row, int plane) {
+  if constexpr (kPair) tc::tma_load_3d_2cta(dst, map, full, k, row, plane);
+  else tc::tma_load_3d(dst, map, full, k, row, plane);
+}
+
+template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kPair>
 __global__ void __launch_bounds__(kThreads, 1)
-    grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                        const __grid_constant__ WeightMaps wmaps,
+    grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
+                        const __grid_constant__ TokenMaps tmap_x,
                         const __grid_constant__ GroupedGemmArgs g) {
+  constexpr int kCtas = kPair ? 2 : 1;
+  constexpr int kUnit = 16 * kCtas;  // steps of an MMA's N: 16, or 32 for M = 256 over a pair
+  constexpr int kCols = SWIGLU ? kBlockM / 2 : kBlockM;  // output columns per CTA and tile
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // Stage ring first (1024-byte aligned tiles), control block and tile table after.
-  uint8_t* stages = reinterpret_cast<uint8_t*>(
+  uint8_t* ring = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  constexpr int kNumStages = kTwoCta ? kStages2 : kStages;
-  constexpr uint32_t kStageStride = kTwoCta ? kStageBytes2 : kStageBytes;
-  SharedControl* ctl = reinterpret_cast<SharedControl*>(stages + kNumStages * kStageStride);
-  // A CTA pair works on one tile of 256 rows; this CTA owns rows [128 * cta_rank, +128).
-  const uint32_t cta_rank = kTwoCta ? tc::cluster_ctarank() : 0u;
-  const bool leader = cta_rank == 0u;
-  const int tile_m = kTwoCta ? 2 * kBlockM : kBlockM;
-  const uint32_t worker = kTwoCta ? blockIdx.x >> 1 : blockIdx.x;   // tile-loop index
-  const uint32_t workers = kTwoCta ? gridDim.x >> 1 : gridDim.x;
+  Control* ctl = reinterpret_cast<Control*>(ring + g.ring_bytes);
+  // (kToPeers only) behind the control block; the tables come last.
+  PeerStage* peer_stage = reinterpret_cast<PeerStage*>(ctl + 1);
+  uint32_t* tile_start = kToPeers ? reinterpret_cast<uint32_t*>(peer_stage + 1)
+                                  : reinterpret_cast<uint32_t*>(ctl + 1);  // [E + 1]
+  uint32_t* rows_of = tile_start + g.num_experts + 1;                      // [E] valid rows
+  uint32_t* x_row0 = rows_of + g.num_experts;  // [E] first row in the token plane
+  // kFromStaging: [E][world] rows that each source sends to the expert, or null when the table
+  // does not fit (then the posted histograms are read again for every tile).
+  uint32_t* src_rows = (kFromStaging && g.src_table != 0) ? x_row0 + g.num_experts : nullptr;
   const A2AParams& p = g.a2a;
-  const int num_groups = g.num_experts;
-  GroupTable gt;
-  gt.tile_start = reinterpret_cast<uint32_t*>(ctl + 1);  // [G + 1]
-  gt.rows = gt.tile_start + num_groups + 1;
-  gt.a_row0 = gt.rows + num_groups;
-  gt.out_row0 = gt.a_row0 + num_groups;
-  gt.src_rows = (kFromStaging && g.src_table != 0) ? gt.out_row0 + num_groups : nullptr;
-  // (kToPeers only) staging of the peer-storing epilogue, behind the tables, 16-byte aligned.
-  PeerStage* peer_stage = reinterpret_cast<PeerStage*>(
-      (reinterpret_cast<uintptr_t>(gt.out_row0 + num_groups) + 15) & ~static_cast<uintptr_t>(15));
+  int parity = 0;
+  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
 
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5;
-  const int lane = tid & 31;
+  const uint32_t cta_rank = kPair ? tc::cluster_ctarank() : 0u;
+  const bool leader = cta_rank == 0u;
+  const uint32_t worker = blockIdx.x / kCtas;   // tile-loop index
+  const uint32_t workers = gridDim.x / kCtas;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile uint32_t* abort_flag = &ctl->abort_flag;
-
+  const int w_blocks = ceil_div<int>(g.n_out, kCols * kCtas);
   const int num_kb = ceil_div<int>(g.k, kBlockK);
 
   // ---- set-up ---------------------------------------------------------------
-  if (tid == 0) ctl->abort_flag = 0;
-  int parity = 0;
-  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
+  if (tid == 0) {
+    ctl->abort_flag = 0;
+    ctl->max_rows = 0;
+    ctl->max_width = kUnit;
+    ctl->best_limit = ~0ull;
+    for (int s = 0; s < kMaxStages; ++s) {
+      tc::mbar_init(&ctl->full[s], 1);
+      tc::mbar_init(&ctl->empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      tc::mbar_init(&ctl->tmem_full[b], 1);
+      tc::mbar_init(&ctl->tmem_empty[b], 8 * kCtas);  // epilogue warps of the tile
+    }
+    tc::fence_mbar_init();
+    tc::tma_prefetch_desc(&tmap_w);
+    tc::tma_prefetch_desc(&tmap_x.x64);
+    tc::tma_prefetch_desc(&tmap_x.x16);
+  }
+  if (warp == 2) {
+    if constexpr (kPair) {
+      tc::tmem_alloc_2cta(&ctl->tmem_base, kTmemCols);
+      tc::tmem_relinquish_2cta();
+    } else {
+      tc::tmem_alloc(&ctl->tmem_base, kTmemCols);
+      tc::tmem_relinquish();
+    }
+  }
   if constexpr (kFromStaging) {
     // Role of the dispatch receive phase: learn how many rows every source sends
     // to every local expert, lay the rows out, publish the per-expert totals.
-    for (int le = tid; le < num_groups; le += blockDim.x) gt.rows[le] = 0;
+    for (int le = tid; le < g.num_experts; le += blockDim.x) rows_of[le] = 0;
     __syncthreads();
     const WaitCtx w{p.status, p.timeout_ns, static_cast<uint32_t>(p.rank)};
     const uint32_t* all = reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_counts_all) +
@@ -221,32 +242,33 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool ok = wait_until(all + static_cast<size_t>(src) * p.num_experts + p.rank * p.nle + le,
                                  PredNonZero{}, v, w, kPhaseDispatchCounts, src, 1u);
       if (!ok) ctl->abort_flag = 1;
-      if (ok && v > 1u) atomicAdd(&gt.rows[le], v - 1u);
-      if (gt.src_rows != nullptr) gt.src_rows[le * p.world + src] = (ok && v > 1u) ? v - 1u : 0u;
+      if (ok && v > 1u) atomicAdd(&rows_of[le], v - 1u);
+      if (src_rows != nullptr) src_rows[le * p.world + src] = (ok && v > 1u) ? v - 1u : 0u;
     }
     __syncthreads();
-    for (int le = tid; le < num_groups; le += blockDim.x) {
-      uint32_t first = 0;
-      for (int l2 = 0; l2 < le; ++l2) first += gt.rows[l2];
-      gt.a_row0[le] = first;
-      gt.out_row0[le] = 0;
-      const uint32_t rows = min(gt.rows[le], static_cast<uint32_t>(p.cap));
-      gt.tile_start[le] = static_cast<uint32_t>(ceil_div<int>(static_cast<int>(rows), tile_m));
-      if (blockIdx.x == 0) {
-        if (g.out_num_tokens != nullptr) g.out_num_tokens[le] = static_cast<int32_t>(gt.rows[le]);
-        p.recv_count[le] = rows;
+    for (int le = tid; le < g.num_experts; le += blockDim.x) x_row0[le] = rows_of[le];
+    __syncthreads();
+    if (warp == 0) warp_exclusive_scan_smem(x_row0, g.num_experts, lane, false);
+    __syncthreads();
+    if (blockIdx.x == 0) {
+      for (int le = tid; le < g.num_experts; le += blockDim.x) {
+        if (g.out_num_tokens != nullptr) g.out_num_tokens[le] = static_cast<int32_t>(rows_of[le]);
+        p.recv_count[le] = min(rows_of[le], static_cast<uint32_t>(p.cap));
       }
     }
-    __syncthreads();
-    for (int le = tid; le < num_groups; le += blockDim.x) gt.rows[le] = min(gt.rows[le], static_cast<uint32_t>(p.cap));
   } else {
-    for (int e = tid; e < num_groups; e += blockDim.x) {
-      const int rows = min(max(g.counts[e], 0), g.rows_per_expert);
-      gt.rows[e] = static_cast<uint32_t>(rows);
-      gt.a_row0[e] = 0;
-      gt.out_row0[e] = 0;
-      gt.tile_start[e] = static_cast<uint32_t>(ceil_div<int>(rows, tile_m));
+    __syncthreads();
+  }
+  for (int e = tid; e < g.num_experts; e += blockDim.x) {
+    int rows;
+    if constexpr (kFromStaging) {
+      rows = static_cast<int>(min(rows_of[e], static_cast<uint32_t>(p.cap)));
+    } else {
+      rows = min(max(g.counts[e], 0), g.rows_per_expert);
+      x_row0[e] = 0;
     }
+    rows_of[e] = static_cast<uint32_t>(rows);
+    if (rows > 0) atomicMax(&ctl->max_rows, static_cast<uint32_t>(rows));
   }
   if constexpr (kToPeers) {
     if (blockIdx.x == 0) {
@@ -263,71 +285,50 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (tid == 0) *p.iter = *p.iter + 1u;
     }
   }
-  if (tid == 0) {
-    for (int s = 0; s < kNumStages; ++s) {
-      tc::mbar_init(&ctl->full[s], 1);
-      tc::mbar_init(&ctl->empty[s], 1);
+  __syncthreads();
+
+  // The most token rows a tile may have.  One tile per expert where that is possible: below
+  // 256 rows an expert is bound by its weights, which more tiles would only read again.  Above,
+  // the limit that minimises (waves of tiles) x (time of a tile); the time of a tile is its
+  // width plus a constant for its barriers and its share of the epilogue.  Every CTA computes
+  // the same.
+  int limit = g.max_tokens / kUnit * kUnit;
+  if (ctl->max_rows > static_cast<uint32_t>(limit)) {
+    for (int cand = limit - kUnit * warp; 2 * cand >= limit; cand -= kUnit * (kThreads / 32)) {
+      uint32_t tiles = 0, width = 0;
+      for (int e = lane; e < g.num_experts; e += 32) {
+        const Cut<kUnit> cut(static_cast<int>(rows_of[e]), cand);
+        tiles += cut.tiles;
+        width += cut.units * kUnit;
+      }
+      tiles = __reduce_add_sync(0xffffffffu, tiles);
+      width = __reduce_add_sync(0xffffffffu, width);
+      if (lane == 0) {
+        const uint64_t waves = ceil_div<uint64_t>(static_cast<uint64_t>(tiles) * w_blocks, workers);
+        const uint64_t cost = waves * (16ull * width / tiles + 16 * kTileOverhead);
+        atomicMin(&ctl->best_limit, (cost << 16) | static_cast<uint64_t>(512 - cand));
+      }
     }
-    for (int b = 0; b < 2; ++b) {
-      tc::mbar_init(&ctl->tmem_full[b], 1);
-      tc::mbar_init(&ctl->tmem_empty[b], kTwoCta ? 8 : 4);  // epilogue warps of the tile
-    }
-    tc::fence_mbar_init();
-    tc::tma_prefetch_desc(&tmap_a);
+    __syncthreads();
+    limit = 512 - static_cast<int>(ctl->best_limit & 0xffffu);
+  }
+  for (int e = tid; e < g.num_experts; e += blockDim.x) {
+    const Cut<kUnit> cut(static_cast<int>(rows_of[e]), limit);
+    tile_start[e] = static_cast<uint32_t>(cut.tiles * w_blocks);
+    if (cut.tiles > 0) atomicMax(&ctl->max_width, static_cast<uint32_t>(cut.widest()));
   }
   __syncthreads();
-  if (warp == 0) warp_exclusive_scan_smem(gt.tile_start, num_groups, lane, true);
-  if (warp == 2) {
-    if constexpr (kTwoCta) {
-      tc::tmem_alloc_2cta(&ctl->tmem_base, kTmemCols);
-      tc::tmem_relinquish_2cta();
-    } else {
-      tc::tmem_alloc(&ctl->tmem_base, kTmemCols);
-      tc::tmem_relinquish();
-    }
-  }
+  if (warp == 0) warp_exclusive_scan_smem(tile_start, g.num_experts, lane, true);
   tc::tc_fence_before_sync();
   __syncthreads();
   // The peer must see initialised barriers before anything arrives on them remotely.
-  if constexpr (kTwoCta) tc::cluster_sync();
+  if constexpr (kPair) tc::cluster_sync();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = ctl->tmem_base;
-
-  // Tile width.  gt.tile_start holds the prefix of ROW blocks per expert; with the
-  // real total the width that minimises (waves of tiles) x (time of one tile) is
-  // chosen among the candidates the host prepared -- every CTA computes the same.
-  // The B tile is two halves of half_n weight rows each (gate and up rows for
-  // SwiGLU, consecutive rows otherwise); the accumulator is 2 * half_n columns wide.
-  const uint32_t total_m_tiles = gt.tile_start[num_groups];
-  int width_idx = 0;
-  {
-    uint64_t best = ~0ull;
-    for (int i = 0; i < kNumTileWidths; ++i) {
-      const int half = g.widths[i];
-      if (half <= 0) continue;
-      const uint32_t nb = ceil_div<uint32_t>(g.n_out, (SWIGLU ? 1 : 2) * half);
-      const uint64_t waves = ceil_div<uint64_t>(static_cast<uint64_t>(total_m_tiles) * nb, workers);
-      const uint64_t cost = waves * static_cast<uint64_t>(half + (kTwoCta ? 40 : 88));
-      if (cost < best) {
-        best = cost;
-        width_idx = i;
-      }
-    }
-  }
-  const CUtensorMap& tmap_b = wmaps.m[width_idx];
-  const int half_n = g.widths[width_idx];
-  const int tile_n = 2 * half_n;
-  const uint32_t b_half_bytes = static_cast<uint32_t>(half_n) * kBlockK * 2;
-  // Bytes that complete one stage: both B halves from this CTA, or (pair) A and one
-  // B half from each of the two CTAs, all counted on the leader's barrier.
-  const uint32_t stage_tx_bytes = kTwoCta ? 2 * (kABytes + b_half_bytes) : kABytes + 2 * b_half_bytes;
-  const int out_cols_per_tile = SWIGLU ? half_n : tile_n;
-  const int n_blocks = ceil_div<int>(g.n_out, out_cols_per_tile);
-  __syncthreads();
-  for (int i = tid; i <= num_groups; i += blockDim.x) gt.tile_start[i] *= static_cast<uint32_t>(n_blocks);
-  __syncthreads();
-  const uint32_t total_tiles = gt.tile_start[num_groups];
-  if (warp == 0 && lane == 0) tc::tma_prefetch_desc(&tmap_b);
+  const uint32_t total_tiles = tile_start[g.num_experts];
+  // As many stages as the launch's widest token tile leaves room for.
+  const uint32_t stage_bytes = kWBytes + ctl->max_width / kCtas * kRowBytes;
+  const uint32_t stages = min(g.ring_bytes / stage_bytes, static_cast<uint32_t>(kMaxStages));
 
   // ---- roles ----------------------------------------------------------------
   if (warp == 0) {
@@ -336,87 +337,52 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t pending = 0;        // stages that have been filled at least once
       uint32_t pending_phase = 0;  // parity of the phase each stage was last filled in
       bool ok = *abort_flag == 0u;
-      int last_group = -1;     // expert that `landed` refers to
-      uint32_t landed = 0;     // bit s: the rows of source s for that expert have landed
+      int last_expert = -1;  // expert that `landed` refers to
+      uint32_t landed = 0;   // bit s: the rows of source s for that expert have landed
       for (uint32_t t = worker; t < total_tiles && ok; t += workers) {
-        const TileCoord c = locate_tile<kFromStaging>(gt, num_groups, p, t, tile_m);
+        const Tile c = locate<kUnit>(tile_start, rows_of, g.num_experts, limit, t);
         if constexpr (kFromStaging) {
-          // The tile's rows were stored by peers.  Wait for the arrival counters of the
-          // sources it covers (rows of an expert are grouped by source rank), then order
-          // the peers' (generic-proxy) stores before the TMA (async-proxy) reads.
-          if (c.group != last_group) {
-            last_group = c.group;
+          if (c.expert != last_expert) {
+            last_expert = c.expert;
             landed = 0;
           }
-          const WaitCtx w{p.status, p.timeout_ns, static_cast<uint32_t>(p.rank)};
-          const uint32_t* arrived =
-              reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_arrived_e) +
-              (static_cast<size_t>(parity) * p.nle + c.group) * p.world;
-          const uint32_t r0 = static_cast<uint32_t>(c.m_blk * tile_m);
-          const uint32_t r1 = min(r0 + static_cast<uint32_t>(tile_m), static_cast<uint32_t>(c.rows));
-          uint32_t first = 0;  // first row of source s inside the expert
-          bool waited = false;
-          for (int s = 0; s < p.world && ok; ++s) {
-            uint32_t n;
-            if (gt.src_rows != nullptr) {
-              n = gt.src_rows[c.group * p.world + s];
-            } else {
-              // No per-source table: counts straight from the posted histograms.
-              const uint32_t v = ptx::ld_relaxed_sys(
-                  reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_counts_all) +
-                  (static_cast<size_t>(parity) * p.world + s) * p.num_experts + p.rank * p.nle +
-                  c.group);
-              n = v > 1u ? v - 1u : 0u;
-            }
-            const bool overlaps = n > 0 && first < r1 && first + n > r0;
-            if (overlaps && !((landed >> s) & 1u)) {
-              uint32_t seen;
-              ok = wait_until(arrived + s, PredGe{n}, seen, w, kPhaseFusedGemm,
-                              static_cast<uint32_t>(s), n);
-              landed |= 1u << s;
-              waited = true;
-            }
-            first += n;
-          }
+          ok = wait_tile_sources(p, c.expert, c.first, min(c.first + c.width, c.rows), parity,
+                                 src_rows, landed);
           if (!ok) {
             *abort_flag = 1u;
             break;
           }
-          if (waited) ptx::fence_proxy_async();
         }
+        const int own = c.width / kCtas;  // this CTA's share of the tokens
+        const int x_row = static_cast<int>(x_row0[c.expert]) + c.first + static_cast<int>(cta_rank) * own;
+        const int x_plane = kFromStaging ? 0 : c.expert;
+        const int w_row = (c.w_blk * kCtas + static_cast<int>(cta_rank)) * kCols;
+        const uint32_t tx = kCtas * (kWBytes + static_cast<uint32_t>(own) * kRowBytes);
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = tc::mbar_wait(&ctl->empty[stage], phase ^ 1u, abort_flag, kWaitLimitNs);
           if (!ok) break;
-          uint8_t* a_dst = stages + stage * kStageStride;
-          uint8_t* b_dst = a_dst + kABytes;
+          uint8_t* w_dst = ring + stage * stage_bytes;
+          uint8_t* x_dst = w_dst + kWBytes;
+          uint64_t* full = &ctl->full[stage];
           pending |= 1u << stage;
           pending_phase = (pending_phase & ~(1u << stage)) | (phase << stage);
-          const int a_row = c.a_row0 + c.m_blk * tile_m + static_cast<int>(cta_rank) * kBlockM;
-          if constexpr (kTwoCta) {
-            // This CTA's rows of A and its half of the weight tile; the bytes of both CTAs
-            // are counted on the leader's barrier, which only the leader arms.
-            if (leader) tc::mbar_arrive_expect_tx(&ctl->full[stage], stage_tx_bytes);
-            int b_row;
-            if constexpr (SWIGLU) b_row = (cta_rank == 0 ? 0 : g.n_out) + c.n_blk * half_n;
-            else b_row = c.n_blk * tile_n + static_cast<int>(cta_rank) * half_n;
-            tc::tma_load_3d_2cta(a_dst, &tmap_a, &ctl->full[stage], kb * kBlockK, a_row, c.a_plane);
-            tc::tma_load_3d_2cta(b_dst, &tmap_b, &ctl->full[stage], kb * kBlockK, b_row, c.w_plane);
+          // The bytes of both CTAs are counted on the leader's barrier, which only the leader
+          // arms.
+          if (leader) tc::mbar_arrive_expect_tx(full, tx);
+          if constexpr (SWIGLU) {
+            if constexpr (kPair)
+              tc::tma_load_5d_2cta(w_dst, &tmap_w, full, kb * kBlockK, 0, 0, w_row / 8, c.expert);
+            else
+              tc::tma_load_5d(w_dst, &tmap_w, full, kb * kBlockK, 0, 0, w_row / 8, c.expert);
           } else {
-            tc::mbar_arrive_expect_tx(&ctl->full[stage], stage_tx_bytes);
-            tc::tma_load_3d(a_dst, &tmap_a, &ctl->full[stage], kb * kBlockK, a_row, c.a_plane);
-            if constexpr (SWIGLU) {
-              const int row = c.n_blk * half_n;
-              tc::tma_load_3d(b_dst, &tmap_b, &ctl->full[stage], kb * kBlockK, row, c.w_plane);
-              tc::tma_load_3d(b_dst + b_half_bytes, &tmap_b, &ctl->full[stage], kb * kBlockK,
-                              g.n_out + row, c.w_plane);
-            } else {
-              const int row = c.n_blk * tile_n;
-              tc::tma_load_3d(b_dst, &tmap_b, &ctl->full[stage], kb * kBlockK, row, c.w_plane);
-              tc::tma_load_3d(b_dst + b_half_bytes, &tmap_b, &ctl->full[stage], kb * kBlockK,
-                              row + half_n, c.w_plane);
-            }
+            load_rows<kPair>(w_dst, &tmap_w, full, kb * kBlockK, w_row, c.expert);
           }
-          if (++stage == kNumStages) {
+          int r = 0;
+          for (; r + 64 <= own; r += 64)
+            load_rows<kPair>(x_dst + r * kRowBytes, &tmap_x.x64, full, kb * kBlockK, x_row + r, x_plane);
+          for (; r < own; r += 16)
+            load_rows<kPair>(x_dst + r * kRowBytes, &tmap_x.x16, full, kb * kBlockK, x_row + r, x_plane);
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -425,16 +391,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok || *abort_flag != 0u) {
         // Give the loads already issued a bounded time to land before the CTA
         // leaves: their destination is this CTA's shared memory.
-        uint64_t t0;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-        for (int s = 0; s < kNumStages; ++s) {
+        const uint64_t t0 = ptx::globaltimer_ns();
+        for (uint32_t s = 0; s < stages; ++s) {
           if (!((pending >> s) & 1u)) continue;
           // (The non-leader of a pair has no barrier of its own to watch; it just sits
           // out the time limit, which is far longer than any load takes.)
           while (!leader || !tc::mbar_try_wait(&ctl->full[s], (pending_phase >> s) & 1u)) {
-            uint64_t t1;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-            if (t1 - t0 > 100000000ull) break;  // 100 ms in total
+            if (ptx::globaltimer_ns() - t0 > 100000000ull) break;  // 100 ms in total
           }
         }
       }
@@ -442,182 +405,164 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncwarp();
   } else if (warp == 1) {
     if (leader && tc::elect_one()) {
-      const uint32_t idesc = tc::make_instr_desc(1u, tile_m, tile_n);
-      uint32_t stage = 0, phase = 0;
-      uint32_t local = 0;
+      uint32_t stage = 0, phase = 0, local = 0;
       bool ok = *abort_flag == 0u;
       for (uint32_t t = worker; t < total_tiles && ok; t += workers, ++local) {
+        const Tile c = locate<kUnit>(tile_start, rows_of, g.num_experts, limit, t);
+        const uint32_t idesc = tc::make_instr_desc(1u, kBlockM * kCtas, c.width);
         const uint32_t buf = local & 1u;
         const uint32_t use = local >> 1;  // how often this accumulator was used before
         ok = tc::mbar_wait(&ctl->tmem_empty[buf], (use & 1u) ^ 1u, abort_flag, kWaitLimitNs);
         if (!ok) break;
         tc::tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + buf * kBlockN;
+        const uint32_t tmem_d = tmem_base + buf * kMaxTokens;
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = tc::mbar_wait(&ctl->full[stage], phase, abort_flag, kWaitLimitNs);
           if (!ok) break;
           tc::tc_fence_after_sync();
-          const uint8_t* a_src = stages + stage * kStageStride;
-          const uint64_t a_desc = tc::make_smem_desc_sw128(a_src);
-          const uint64_t b_desc = tc::make_smem_desc_sw128(a_src + kABytes);
+          const uint8_t* w_src = ring + stage * stage_bytes;
+          const uint64_t w_desc = tc::make_smem_desc_sw128(w_src);
+          const uint64_t x_desc = tc::make_smem_desc_sw128(w_src + kWBytes);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k) {
-            if constexpr (kTwoCta) {
-              tc::mma_f16_ss_2cta(tmem_d, tc::advance_smem_desc(a_desc, k * kUmmaK * 2),
-                                  tc::advance_smem_desc(b_desc, k * kUmmaK * 2), idesc,
-                                  (kb | k) != 0);
-            } else {
-              tc::mma_f16_ss(tmem_d, tc::advance_smem_desc(a_desc, k * kUmmaK * 2),
-                             tc::advance_smem_desc(b_desc, k * kUmmaK * 2), idesc,
-                             (kb | k) != 0);
-            }
+            const uint64_t wd = tc::advance_smem_desc(w_desc, k * kUmmaK * 2);
+            const uint64_t xd = tc::advance_smem_desc(x_desc, k * kUmmaK * 2);
+            if constexpr (kPair) tc::mma_f16_ss_2cta(tmem_d, wd, xd, idesc, (kb | k) != 0);
+            else tc::mma_f16_ss(tmem_d, wd, xd, idesc, (kb | k) != 0);
           }
           // Stage reusable (in both CTAs of a pair) once these MMAs have read it.
-          if constexpr (kTwoCta) tc::mma_commit_2cta(&ctl->empty[stage], 0x3);
+          if constexpr (kPair) tc::mma_commit_2cta(&ctl->empty[stage], 0x3);
           else tc::mma_commit(&ctl->empty[stage]);
-          if (++stage == kNumStages) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (ok) {
-          if constexpr (kTwoCta) tc::mma_commit_2cta(&ctl->tmem_full[buf], 0x3);
+          if constexpr (kPair) tc::mma_commit_2cta(&ctl->tmem_full[buf], 0x3);
           else tc::mma_commit(&ctl->tmem_full[buf]);
         }
       }
     }
     __syncwarp();
   } else if (warp >= 4) {
-    const int ew = warp - 4;  // lanes [32 * ew, 32 * ew + 32) of tensor memory
+    const int ew = (warp - 4) & 3;   // tensor-memory lanes [32 * ew, +32)
+    const int wg = (warp - 4) >> 2;  // 16-token groups wg, wg + 2, wg + 4, ...
+    const int n_tid = tid - 128;     // 0..255 over the eight warps
+    const int lt = n_tid & 127;      // thread of the warp group
+    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(ew * 32) << 16);
     uint32_t local = 0;
+    uint32_t pending_signals = 0;  // kToPeers, warp 4: queued arrival adds
     bool ok = *abort_flag == 0u;
-    const int row_bytes_out = g.n_out * 2;
     for (uint32_t t = worker; t < total_tiles && ok; t += workers, ++local) {
-      const TileCoord c = locate_tile<kFromStaging>(gt, num_groups, p, t, tile_m);
+      const Tile c = locate<kUnit>(tile_start, rows_of, g.num_experts, limit, t);
       const uint32_t buf = local & 1u;
-      const uint32_t use = local >> 1;
-      ok = tc::mbar_wait(&ctl->tmem_full[buf], use & 1u, abort_flag, kWaitLimitNs);
+      ok = tc::mbar_wait(&ctl->tmem_full[buf], (local >> 1) & 1u, abort_flag, kWaitLimitNs);
+      // All eight warps leave together or not at all: the barriers below must never be
+      // entered by only some of them.
+      {
+        uint32_t all_ok;
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p, q;\n\t"
+            "setp.ne.u32 q, %1, 0;\n\t"
+            "bar.red.and.pred p, 1, 256, q;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t"
+            "}\n"
+            : "=r"(all_ok)
+            : "r"(ok ? 1u : 0u)
+            : "memory");
+        ok = all_ok != 0u;
+      }
       if (!ok) break;
       tc::tc_fence_after_sync();
-      const int tile_row = ew * 32 + lane;
-      const int row = c.m_blk * tile_m + static_cast<int>(cta_rank) * kBlockM + tile_row;
-      const bool row_ok = row < c.rows;
-      const int out_row = c.out_row0 + row;
-
-      // Where this thread's row goes.
-      __nv_bfloat16* local_row = nullptr;
-      size_t peer_off = 0;
-      const int replicas = kToPeers ? min(p.dp_size, 8) : 0;
-      uint32_t sig_token = kNoSignal, sig_group = 0;
-      if constexpr (kToPeers) {
-        if (row_ok) {
-          const uint2 rs = p.row_src[static_cast<size_t>(c.w_plane) * p.cap + out_row];
-          const int src_rank = static_cast<int>(rs.x & 0xffffu);
-          const uint32_t k = rs.x >> 16;
-          const uint32_t token = rs.y;
-          if (token < static_cast<uint32_t>(p.max_tokens) && k < static_cast<uint32_t>(p.topk) &&
-              src_rank < p.world) {
-            sig_token = token;
-            sig_group = static_cast<uint32_t>((src_rank / p.dp_size) * p.dp_size);
-            peer_off = p.off_comb_stage + (static_cast<size_t>(token) * p.topk + k) * row_bytes_out;
-          } else if (p.debug_checks) {
-            report_failure(p.status, kBadToken, kPhaseCombinePayload, src_rank, p.max_tokens,
-                           token, p.rank);
-          }
-        }
-      } else {
-        local_row = g.out + static_cast<int64_t>(c.w_plane) * g.out_stride_e +
-                    static_cast<int64_t>(out_row) * g.out_stride_row;
-      }
+      const int groups = c.width >> 4;
+      const int live = min(c.width, c.rows - c.first);  // tokens of the tile that exist
+      const int col0 = (c.w_blk * kCtas + static_cast<int>(cta_rank)) * kCols;
       if constexpr (kFromStaging) {
-        // First column block of a row also records where the row came from.
-        if (row_ok && c.n_blk == 0) {
+        // The first block of columns also records where the rows came from.
+        if (col0 == 0 && n_tid < live) {
+          const int row = c.first + n_tid;
           const uint8_t* slot = p.peer[p.rank] + p.off_disp_stage +
-                                static_cast<size_t>(c.a_row0 + row) * p.slot_bytes;
+                                (static_cast<size_t>(x_row0[c.expert]) + row) * p.slot_bytes;
           const int4 tr = ptx::ld_cg_v4(slot + p.trailer_off);
           uint2 rs;
           rs.x = (static_cast<uint32_t>(tr.w) & 0xffffu) | (static_cast<uint32_t>(tr.y) << 16);
           rs.y = static_cast<uint32_t>(tr.x);
-          p.row_src[static_cast<size_t>(c.w_plane) * p.cap + out_row] = rs;
+          p.row_src[static_cast<size_t>(c.expert) * p.cap + row] = rs;
         }
       }
-
       if constexpr (kToPeers) {
-        // The rows' destinations, for the lanes that will store other rows' segments and for
-        // the signalling below.  (Double buffered by accumulator; the barrier at the end of
-        // every tile keeps the epilogue warps within one tile of each other.)
-        ctl->sig_token[buf][tile_row] = sig_token;
-        ctl->sig_group[buf][tile_row] = sig_group;
-        peer_stage->row_off[buf][tile_row] = peer_off;
-        __syncwarp();
-      }
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + buf * kBlockN;
-      const int col0 = c.n_blk * out_cols_per_tile;
-#pragma unroll 1
-      for (int chunk = 0; chunk * 32 < out_cols_per_tile; ++chunk) {
-        uint32_t acc[32];
-        uint32_t packed[16];
-        tc::tmem_ld_32x32(taddr + chunk * 32, acc);
-        if constexpr (SWIGLU) {
-          uint32_t up[32];
-          tc::tmem_ld_32x32(taddr + half_n + chunk * 32, up);
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float g0 = __uint_as_float(acc[2 * j]), g1 = __uint_as_float(acc[2 * j + 1]);
-            const float u0 = __uint_as_float(up[2 * j]), u1 = __uint_as_float(up[2 * j + 1]);
-            packed[j] = pack_bf16(silu(g0) * u0, silu(g1) * u1);
-          }
-        } else {
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            packed[j] = pack_bf16(__uint_as_float(acc[2 * j]), __uint_as_float(acc[2 * j + 1]));
-          }
-        }
-        const int col = col0 + chunk * 32;
-        if constexpr (kToPeers) {
-          uint8_t* stg = &peer_stage->rows[ew][0][0];
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            int4 q;
-            q.x = packed[4 * v];
-            q.y = packed[4 * v + 1];
-            q.z = packed[4 * v + 2];
-            q.w = packed[4 * v + 3];
-            *reinterpret_cast<int4*>(stg + lane * kOutStageRowBytes + (chunk & 1) * 64 + v * 16) = q;
-          }
-          const bool last_chunk = (chunk + 1) * 32 >= out_cols_per_tile;
-          if ((chunk & 1) == 1 || last_chunk) {
-            __syncwarp();
-            const int pair0 = (chunk & ~1) * 32;  // first tile column of the staged pair
-            const int seg = lane & 7;             // 16-byte piece of the row's 128 bytes
-            const int tcol = pair0 + seg * 8;
-            const bool seg_ok = seg * 8 < ((chunk & 1) + 1) * 32 && tcol + 8 <= out_cols_per_tile &&
-                                col0 + tcol + 8 <= g.n_out;
-#pragma unroll 2
-            for (int it = 0; it < 8; ++it) {
-              const int rr = it * 4 + (lane >> 3);
-              const int trow = ew * 32 + rr;
-              if (seg_ok && ctl->sig_token[buf][trow] != kNoSignal) {
-                const int4 q = *reinterpret_cast<const int4*>(stg + rr * kOutStageRowBytes + seg * 16);
-                const uint32_t grp = ctl->sig_group[buf][trow];
-                const size_t off = peer_stage->row_off[buf][trow] + static_cast<size_t>(col0 + tcol) * 2;
-                for (int r = 0; r < replicas; ++r) ptx::st_v4(p.peer[grp + r] + off, q);
-              }
+        // Where each token's row goes, and whose token it is.  (The barrier above comes after
+        // the last use of the previous tile's table.)
+        if (n_tid < c.width) {
+          unsigned long long off = 0;
+          uint32_t sig_token = kNoSignal, sig_group = 0;
+          if (n_tid < live) {
+            const uint2 rs = p.row_src[static_cast<size_t>(c.expert) * p.cap + c.first + n_tid];
+            const int src_rank = static_cast<int>(rs.x & 0xffffu);
+            const uint32_t k = rs.x >> 16;
+            const uint32_t token = rs.y;
+            if (token < static_cast<uint32_t>(p.max_tokens) && k < static_cast<uint32_t>(p.topk) &&
+                src_rank < p.world) {
+              sig_token = token;
+              sig_group = static_cast<uint32_t>((src_rank / p.dp_size) * p.dp_size);
+              off = p.off_comb_stage +
+                    (static_cast<size_t>(token) * p.topk + k) * (static_cast<size_t>(g.n_out) * 2);
+            } else if (p.debug_checks) {
+              report_failure(p.status, kBadToken, kPhaseCombinePayload, src_rank, p.max_tokens,
+                             token, p.rank);
             }
-            __syncwarp();
           }
+          peer_stage->token[n_tid] = sig_token;
+          peer_stage->group[n_tid] = sig_group;
+          peer_stage->row_off[n_tid] = off;
+        }
+        asm volatile("bar.sync 4, 256;" ::: "memory");
+      }
+      // A thread's values lie across token rows; each group of 16 tokens passes through shared
+      // memory so that rows leave in 16-byte pieces.
+      const uint32_t t_acc = t_lane + buf * kMaxTokens;
+#pragma unroll 1
+      for (int grp = wg, alt = 0; grp < groups; grp += 2, alt ^= 1) {
+        uint32_t lo[8], hi[8];
+        load_group(t_acc + grp * 16, lo, hi);
+        tc::tmem_ld_wait();
+        uint8_t(*seg)[kSegBytes] = ctl->seg[wg][alt];
+        if constexpr (SWIGLU) {
+          // Lanes 0-7 of every 16 are gate rows, 8-15 the up rows of the same columns.
+          stmatrix_x4_trans(&seg[8 * (lane >> 4) + (lane & 7)][(ew * 16 + ((lane >> 3) & 1) * 8) * 2],
+                            swiglu_pair(lo[0], lo[1], lo[2], lo[3]),
+                            swiglu_pair(hi[0], hi[1], hi[2], hi[3]),
+                            swiglu_pair(lo[4], lo[5], lo[6], lo[7]),
+                            swiglu_pair(hi[4], hi[5], hi[6], hi[7]));
         } else {
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            if (chunk * 32 + v * 8 + 8 > out_cols_per_tile || col + v * 8 + 8 > g.n_out) continue;
-            int4 q;
-            q.x = packed[4 * v];
-            q.y = packed[4 * v + 1];
-            q.z = packed[4 * v + 2];
-            q.w = packed[4 * v + 3];
-            if (row_ok) *reinterpret_cast<int4*>(local_row + col + v * 8) = q;
+          for (int b = 0; b < 2; ++b)
+            stmatrix_x4_trans(&seg[8 * b + (lane & 7)][(ew * 32 + (lane >> 3) * 8) * 2],
+                              pack_bits(lo[4 * b], lo[4 * b + 1]),
+                              pack_bits(lo[4 * b + 2], lo[4 * b + 3]),
+                              pack_bits(hi[4 * b], hi[4 * b + 1]),
+                              pack_bits(hi[4 * b + 2], hi[4 * b + 3]));
+        }
+        sync_group(wg);
+        constexpr int kPieces = kCols / 8;  // 16-byte pieces of a token's row segment
+        const int piece = lt % kPieces;
+        const int col = col0 + piece * 8;
+#pragma unroll
+        for (int tok16 = lt / kPieces; tok16 < 16; tok16 += 128 / kPieces) {
+          const int n = grp * 16 + tok16;
+          const int4 v = *reinterpret_cast<const int4*>(&seg[tok16][piece * 16]);
+          if (col + 8 > g.n_out) continue;
+          if constexpr (kToPeers) {
+            if (peer_stage->token[n] != kNoSignal) {
+              const uint32_t first_rank = peer_stage->group[n];
+              const size_t off = peer_stage->row_off[n] + static_cast<size_t>(col) * 2;
+              for (int r = 0; r < min(p.dp_size, 8); ++r) ptx::st_v4(p.peer[first_rank + r] + off, v);
+            }
+          } else if (n < live) {
+            *reinterpret_cast<int4*>(g.out + c.expert * g.out_stride_e +
+                                     static_cast<int64_t>(c.first + n) * g.out_stride_row + col) = v;
           }
         }
       }
@@ -625,28 +570,37 @@ __global__ void __launch_bounds__(kThreads, 1)
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        if constexpr (kTwoCta) tc::mbar_arrive_on_leader(&ctl->tmem_empty[buf]);
+        if constexpr (kPair) tc::mbar_arrive_on_leader(&ctl->tmem_empty[buf]);
         else tc::mbar_arrive(&ctl->tmem_empty[buf]);
       }
-
       if constexpr (kToPeers) {
-        // One fence for the whole tile, then the adds.
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (ew == 0) {
-          ptx::fence_acq_rel_sys();
-          // Arrival is counted in columns: this tile's share of the row.
-          const uint32_t units = static_cast<uint32_t>(min(out_cols_per_tile, g.n_out - col0));
-          for (int j = lane; j < kBlockM; j += 32) {
-            const uint32_t tok = ctl->sig_token[buf][j];
-            if (tok == kNoSignal) continue;
-            const uint32_t grp = ctl->sig_group[buf][j];
-            for (int r = 0; r < min(p.dp_size, 8); ++r) {
-              ptx::red_add_relaxed_sys(
-                  reinterpret_cast<uint32_t*>(p.peer[grp + r] + p.off_comb_arrived) + tok, units);
-            }
+        // Arrival is counted in columns: this tile's share of each row.  The adds are queued
+        // and flushed behind ONE system-scope fence for as many tiles as the queue holds.
+        asm volatile("bar.sync 4, 256;" ::: "memory");
+        if (warp == 4 && col0 < g.n_out) {
+          const uint32_t units = static_cast<uint32_t>(min(kCols, g.n_out - col0));
+          if (pending_signals + c.width > kQueue) {
+            flush(p, peer_stage, pending_signals, lane);
+            pending_signals = 0;
           }
+          for (int j0 = 0; j0 < c.width; j0 += 32) {
+            const uint32_t token = j0 + lane < c.width ? peer_stage->token[j0 + lane] : kNoSignal;
+            const bool there = token != kNoSignal;
+            const uint32_t mask = __ballot_sync(0xffffffffu, there);
+            if (there) {
+              const uint32_t at = pending_signals + __popc(mask & ((1u << lane) - 1u));
+              peer_stage->q_token[at] = token;
+              peer_stage->q_group_units[at] = peer_stage->group[j0 + lane] | (units << 8);
+            }
+            pending_signals += __popc(mask);
+          }
+          __syncwarp();
         }
       }
+    }
+    if constexpr (kToPeers) {
+      // What is still queued (also after a failed wait: rows that were stored are announced).
+      if (warp == 4 && pending_signals > 0) flush(p, peer_stage, pending_signals, lane);
     }
   }
 
@@ -655,10 +609,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   // Neither CTA of a pair may leave while the other can still touch its shared or
   // tensor memory.
-  if constexpr (kTwoCta) tc::cluster_sync();
+  if constexpr (kPair) tc::cluster_sync();
   if (warp == 2) {
     tc::tc_fence_after_sync();
-    if constexpr (kTwoCta) tc::tmem_dealloc_2cta(tmem_base, kTmemCols);
+    if constexpr (kPair) tc::tmem_dealloc_2cta(tmem_base, kTmemCols);
     else tc::tmem_dealloc(tmem_base, kTmemCols);
   }
   if (tid == 0 && ctl->abort_flag != 0u && g.status != nullptr) *g.status = 1u;
@@ -682,87 +636,105 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// [experts, rows, k] bf16 with k contiguous; tiles of 64 x 128 x 1, 128-byte swizzle,
-// out-of-range elements read as zero.
-CUtensorMap make_operand_map(const void* base, int64_t experts, int64_t rows, int64_t k,
-                             int64_t stride_row_elems, int64_t stride_expert_elems,
-                             int box_rows = 128) {
+CUtensorMap encode_map(int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                       const cuuint32_t* box) {
   PPLX_CHECK(reinterpret_cast<uintptr_t>(base) % 16 == 0, "operand base must be 16-byte aligned");
-  PPLX_CHECK((stride_row_elems * 2) % 16 == 0 && (stride_expert_elems * 2) % 16 == 0,
-             "operand strides must be multiples of 16 bytes (8 bf16 elements)");
+  const cuuint32_t elem_strides[5] = {1, 1, 1, 1, 1};
   CUtensorMap map;
-  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows),
-                              static_cast<cuuint64_t>(experts)};
-  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(stride_row_elems) * 2,
-                                 static_cast<cuuint64_t>(stride_expert_elems) * 2};
-  const cuuint32_t box[3] = {kBlockK, static_cast<cuuint32_t>(box_rows), 1};
-  const cuuint32_t elem_strides[3] = {1, 1, 1};
   const CUresult r = encode_tiled()(
-      &map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
+      &map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box,
       elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   PPLX_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code " << static_cast<int>(r));
   return map;
 }
 
-// `src_entries`: entries of the per-source row table of the staging-fed form (0: none);
-// `to_peers`: room for the peer-storing epilogue's staging.
-size_t smem_bytes(int num_groups, size_t src_entries = 0, bool to_peers = false) {
-  static_assert(kStages * kStageBytes == kStages2 * kStageBytes2, "both rings use 192 KiB");
-  return 1024 + kStages * kStageBytes + sizeof(SharedControl) +
-         sizeof(uint32_t) * (4 * static_cast<size_t>(num_groups) + 1 + src_entries) +
-         (to_peers ? sizeof(PeerStage) + 16 : 0);
+void check_strides(int64_t stride_row_elems, int64_t stride_expert_elems) {
+  PPLX_CHECK((stride_row_elems * 2) % 16 == 0 && (stride_expert_elems * 2) % 16 == 0,
+             "operand strides must be multiples of 16 bytes (8 bf16 elements)");
+}
+
+// [planes, rows, k] bf16 with k contiguous; tiles of 64 x box_rows x 1, 128-byte swizzle,
+// out-of-range elements read as zero.
+CUtensorMap make_operand_map(const void* base, int64_t planes, int64_t rows, int64_t k,
+                             int64_t stride_row_elems, int64_t stride_plane_elems, int box_rows) {
+  check_strides(stride_row_elems, stride_plane_elems);
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows),
+                              static_cast<cuuint64_t>(planes)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(stride_row_elems) * 2,
+                                 static_cast<cuuint64_t>(stride_plane_elems) * 2};
+  const cuuint32_t box[3] = {kBlockK, static_cast<cuuint32_t>(box_rows), 1};
+  return encode_map(3, base, dims, strides, box);
+}
+
+// 128 weight rows per tile.  Plain: consecutive ones.  SwiGLU: [experts][2 * n_out][k] seen as
+// [experts][n_out / 8][gate, up][8][k], so that a box of 8 x 2 x 8 rows is eight gate rows, the
+// eight up rows of the same columns, the next eight gate rows, ...
+CUtensorMap make_weight_map(const GroupedGemmCall& c) {
+  if (!c.swiglu)
+    return make_operand_map(c.w, c.num_experts, c.n_out, c.k, c.w_stride_row, c.w_stride_e, kBlockM);
+  check_strides(c.w_stride_row, c.w_stride_e);
+  const cuuint64_t row = static_cast<cuuint64_t>(c.w_stride_row) * 2;
+  const cuuint64_t dims[5] = {static_cast<cuuint64_t>(c.k), 8, 2,
+                              static_cast<cuuint64_t>(c.n_out / 8),
+                              static_cast<cuuint64_t>(c.num_experts)};
+  const cuuint64_t strides[4] = {row, row * static_cast<cuuint64_t>(c.n_out), row * 8,
+                                 static_cast<cuuint64_t>(c.w_stride_e) * 2};
+  const cuuint32_t box[5] = {kBlockK, 8, 2, 8, 1};
+  return encode_map(5, c.w, dims, strides, box);
+}
+
+TokenMaps make_token_maps(const void* base, int64_t planes, int64_t rows, int64_t k,
+                          int64_t stride_row, int64_t stride_plane) {
+  return {make_operand_map(base, planes, rows, k, stride_row, stride_plane, 64),
+          make_operand_map(base, planes, rows, k, stride_row, stride_plane, 16)};
 }
 
 // The per-source table is kept in shared memory when it is at most this many entries.
 constexpr size_t kMaxSrcEntries = 2048;
 
-template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kTwoCta>
-void launch_one(const CUtensorMap& tmap_a, const WeightMaps& tmap_b, const GroupedGemmArgs& g,
-                int num_groups, int grid, cudaStream_t stream) {
-  auto* kernel = grouped_gemm_kernel<SWIGLU, kFromStaging, kToPeers, kTwoCta>;
+template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kPair>
+void launch_one(const CUtensorMap& tmap_w, const TokenMaps& tmap_x, GroupedGemmArgs g, int grid,
+                cudaStream_t stream) {
+  auto* kernel = grouped_gemm_kernel<SWIGLU, kFromStaging, kToPeers, kPair>;
   const size_t src_entries =
-      (kFromStaging && g.src_table != 0) ? static_cast<size_t>(num_groups) * g.a2a.world : 0;
-  const size_t smem = smem_bytes(num_groups, src_entries, kToPeers);
-  PPLX_CHECK(smem <= 227 * 1024, "the tile tables of " << num_groups << " experts need " << smem
-                                                       << " bytes of shared memory");
+      (kFromStaging && g.src_table != 0) ? static_cast<size_t>(g.num_experts) * g.a2a.world : 0;
+  const size_t fixed = 1024 + sizeof(Control) + (kToPeers ? sizeof(PeerStage) : 0) +
+                       sizeof(uint32_t) * (3 * static_cast<size_t>(g.num_experts) + 1 + src_entries);
+  // The stages take what the tables leave; kMaxExperts and kMaxSrcEntries leave room for at
+  // least three of the widest tiles.
+  constexpr size_t kSmem = 227 * 1024;
+  static_assert(kSmem - (1024 + sizeof(Control) + sizeof(PeerStage) +
+                         sizeof(uint32_t) * (3 * kMaxExperts + 1 + kMaxSrcEntries)) >=
+                    3 * (kWBytes + kMaxTokens * kRowBytes) + 1024,
+                "too little shared memory for the stages");
+  g.ring_bytes = static_cast<uint32_t>((kSmem - fixed) & ~static_cast<size_t>(1023));
+  const size_t smem = fixed + g.ring_bytes;
   CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(kTwoCta ? (grid & ~1) : grid);
+  cfg.gridDim = dim3(kPair ? (grid & ~1) : grid);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = kTwoCta ? 2 : 1;
+  attr.val.clusterDim.x = kPair ? 2 : 1;
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, tmap_a, tmap_b, g));
+  CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, tmap_w, tmap_x, g));
 }
 
 template <bool SWIGLU, bool kFromStaging, bool kToPeers>
-void launch_variant(const CUtensorMap& tmap_a, const WeightMaps& tmap_b,
-                    const GroupedGemmArgs& g, int num_groups, int grid, bool two_cta,
-                    cudaStream_t stream) {
-  if (two_cta && grid >= 2) {
-    launch_one<SWIGLU, kFromStaging, kToPeers, true>(tmap_a, tmap_b, g, num_groups, grid, stream);
-  } else {
-    launch_one<SWIGLU, kFromStaging, kToPeers, false>(tmap_a, tmap_b, g, num_groups, grid, stream);
-  }
-}
-
-// A CTA pair is ~15 % faster per flop, but an expert's last 256-row tile wastes up
-// to 256 rows of MMA work (128 for single CTAs).  With rows per expert only known
-// on the device, the pair form is chosen when that worst case stays small.
-bool want_two_cta(const GroupedGemmCall& c) {
-  if (c.cta_pair >= 0) return c.cta_pair != 0;
-  const int64_t rows = c.expected_total_rows > 0
-                           ? c.expected_total_rows
-                           : static_cast<int64_t>(c.num_experts) * c.rows_per_expert;
-  return rows / std::max(1, c.num_experts) >= 2048;
+void launch_variant(const CUtensorMap& tmap_w, const TokenMaps& tmap_x, const GroupedGemmArgs& g,
+                    const GroupedGemmCall& c, cudaStream_t stream) {
+  const int grid = c.num_sms > 0 ? c.num_sms : get_sm_count();
+  if (c.cta_pair != 0 && grid >= 2)
+    launch_one<SWIGLU, kFromStaging, kToPeers, true>(tmap_w, tmap_x, g, grid, stream);
+  else
+    launch_one<SWIGLU, kFromStaging, kToPeers, false>(tmap_w, tmap_x, g, grid, stream);
 }
 
 void check_common(const GroupedGemmCall& c) {
@@ -784,30 +756,8 @@ GroupedGemmArgs base_args(const GroupedGemmCall& c) {
   g.rows_per_expert = c.rows_per_expert;
   g.n_out = c.n_out;
   g.k = c.k;
+  g.max_tokens = c.half_n > 0 ? 2 * c.half_n : kMaxTokens;
   return g;
-}
-
-// Candidate tile widths (weight rows per B half) and one weight map for each.  A
-// forced width leaves a single candidate; `units` > 0 (peer-storing epilogue) keeps
-// only the widths whose column-block count divides the arrival units of a row.
-WeightMaps weight_maps(const GroupedGemmCall& c, GroupedGemmArgs& g, int units) {
-  static const int kCandidates[kNumTileWidths] = {128, 112, 96, 80, 64};
-  const int64_t w_rows = c.swiglu ? 2 * static_cast<int64_t>(c.n_out) : c.n_out;
-  WeightMaps maps{};
-  int valid = 0;
-  for (int i = 0; i < kNumTileWidths; ++i) {
-    int half = kCandidates[i];
-    if (c.half_n > 0) half = (i == 0) ? c.half_n : 0;
-    if (half > 0 && units > 0 && units % ceil_div(c.n_out, 2 * half) != 0) half = 0;
-    g.widths[i] = half;
-    // Unused slots still need a well-formed map.
-    maps.m[i] = make_operand_map(c.w, c.num_experts, w_rows, c.k, c.w_stride_row, c.w_stride_e,
-                                 half > 0 ? half : 128);
-    valid += half > 0;
-  }
-  PPLX_CHECK(valid > 0, "no tile width fits: the arrival units of a row ("
-                            << units << ") must be a multiple of the output's column blocks");
-  return maps;
 }
 
 }  // namespace
@@ -817,14 +767,12 @@ void launch_grouped_gemm(const GroupedGemmCall& c, cudaStream_t stream) {
   PPLX_CHECK(reinterpret_cast<uintptr_t>(c.out) % 16 == 0 && c.out_stride_row % 8 == 0 &&
                  c.out_stride_e % 8 == 0,
              "the output must be 16-byte aligned");
-  const CUtensorMap tmap_a = make_operand_map(c.x, c.num_experts, c.rows_per_expert, c.k,
+  const TokenMaps tmap_x = make_token_maps(c.x, c.num_experts, c.rows_per_expert, c.k,
                                               c.x_stride_row, c.x_stride_e);
-  const int grid = c.num_sms > 0 ? c.num_sms : get_sm_count();
-  const bool two_cta = want_two_cta(c);
   GroupedGemmArgs g = base_args(c);
-  const WeightMaps tmap_b = weight_maps(c, g, 0);
-  if (c.swiglu) launch_variant<true, false, false>(tmap_a, tmap_b, g, c.num_experts, grid, two_cta, stream);
-  else launch_variant<false, false, false>(tmap_a, tmap_b, g, c.num_experts, grid, two_cta, stream);
+  const CUtensorMap tmap_w = make_weight_map(c);
+  if (c.swiglu) launch_variant<true, false, false>(tmap_w, tmap_x, g, c, stream);
+  else launch_variant<false, false, false>(tmap_w, tmap_x, g, c, stream);
 }
 
 void launch_gemm_from_staging(const GroupedGemmCall& c, const A2AParams& p,
@@ -838,19 +786,17 @@ void launch_gemm_from_staging(const GroupedGemmCall& c, const A2AParams& p,
   PPLX_CHECK(reinterpret_cast<uintptr_t>(c.out) % 16 == 0 && c.out_stride_row % 8 == 0 &&
                  c.out_stride_e % 8 == 0,
              "the output must be 16-byte aligned");
-  // A: [1][world * region_slots][hidden] bf16 view of this rank's packed staging.
+  // Tokens: [1][world * region_slots][hidden] bf16 view of this rank's packed staging.
   const int64_t slots = static_cast<int64_t>(p.world) * p.region_slots;
-  const CUtensorMap tmap_a = make_operand_map(p.peer[p.rank] + p.off_disp_stage, 1, slots,
+  const TokenMaps tmap_x = make_token_maps(p.peer[p.rank] + p.off_disp_stage, 1, slots,
                                               p.hidden_dim, p.slot_bytes / 2,
                                               slots * p.slot_bytes / 2);
-  const int grid = c.num_sms > 0 ? c.num_sms : get_sm_count();
-  const bool two_cta = want_two_cta(c);
   GroupedGemmArgs g = base_args(c);
-  const WeightMaps tmap_b = weight_maps(c, g, 0);
+  const CUtensorMap tmap_w = make_weight_map(c);
   g.out_num_tokens = out_num_tokens;
   g.a2a = p;
   g.src_table = static_cast<size_t>(p.nle) * p.world <= kMaxSrcEntries ? 1 : 0;
-  launch_variant<true, true, false>(tmap_a, tmap_b, g, p.nle, grid, two_cta, stream);
+  launch_variant<true, true, false>(tmap_w, tmap_x, g, c, stream);
 }
 
 void launch_gemm_to_peers(const GroupedGemmCall& c, const A2AParams& p, cudaStream_t stream) {
@@ -860,16 +806,14 @@ void launch_gemm_to_peers(const GroupedGemmCall& c, const A2AParams& p, cudaStre
              "shape mismatch between the GEMM and the all-to-all");
   PPLX_CHECK(c.counts == reinterpret_cast<const int32_t*>(p.recv_count),
              "counts must be the all-to-all's received-row counts");
-  const int grid = c.num_sms > 0 ? c.num_sms : get_sm_count();
-  const bool two_cta = want_two_cta(c);
   PPLX_CHECK(p.dp_size <= 8, "at most 8 replicas per DP group");
-  const CUtensorMap tmap_a = make_operand_map(c.x, c.num_experts, c.rows_per_expert, c.k,
+  const TokenMaps tmap_x = make_token_maps(c.x, c.num_experts, c.rows_per_expert, c.k,
                                               c.x_stride_row, c.x_stride_e);
   GroupedGemmArgs g = base_args(c);
-  const WeightMaps tmap_b = weight_maps(c, g, 0);
+  const CUtensorMap tmap_w = make_weight_map(c);
   g.out = nullptr;
   g.a2a = p;
-  launch_variant<false, false, true>(tmap_a, tmap_b, g, c.num_experts, grid, two_cta, stream);
+  launch_variant<false, false, true>(tmap_w, tmap_x, g, c, stream);
 }
 
 }  // namespace pplx

@@ -84,7 +84,7 @@ class MoELayer:
         if out is None:
             out = torch.empty(self.max_num_tokens, self.cfg.hidden_dim, dtype=torch.bfloat16,
                               device=self.device)
-        # Rows this rank expects under uniform routing: steers the GEMM tile width only.
+        # Rows this rank expects under uniform routing (a hint; the kernels read the real counts).
         expect = x.size(0) * self.cfg.experts_per_token * (self.world_size // self.dp_size) \
             // self.world_size
         if fused:

@@ -22,11 +22,12 @@ def grouped_gemm(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor,
                  half_n: int = 0, cta_pair: int = -1) -> torch.Tensor:
     """x: [E, rows, K] bf16, w: [E, N or 2N, K] bf16, counts: [E] int32 -> out [E, rows, N] bf16.
 
-    ``expected_rows`` (total valid rows, 0 = capacity) and ``half_n`` (0 = choose) steer the
-    tile width: the accumulator is ``2 * half_n`` columns wide and the launcher picks the
-    width that fills the last wave of tiles best.  ``cta_pair`` selects the kernel form:
-    1 = two CTAs share a 256-row tile (tcgen05 ``cta_group::2``, less shared-memory traffic
-    per flop), 0 = one CTA per 128-row tile, -1 = choose from the expected rows per expert.
+    ``half_n`` (0 = 128) limits a tile to ``2 * half_n`` token rows, the columns of its
+    accumulator; up to that limit the kernel picks the number of tiles from the row counts it
+    reads on the device, so ``expected_rows`` is only kept for callers that pass it.
+    ``cta_pair`` selects the kernel form: 0 = one CTA per tile of 128 weight rows, otherwise two
+    CTAs share a tile of 256 weight rows (tcgen05 ``cta_group::2``, less traffic into shared
+    memory per flop).
     """
     n_out = w.size(1) // 2 if swiglu else w.size(1)
     if out is None:
