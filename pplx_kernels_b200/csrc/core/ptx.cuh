@@ -207,5 +207,19 @@ __device__ __forceinline__ void nanosleep(uint32_t ns) {
   asm volatile("nanosleep.u32 %0;" ::"r"(ns));
 }
 
+// Kernels of one stream that follow each other (launch_after_previous on the host).  The wait
+// returns when every kernel in front of this one has finished and its writes are visible;
+// nothing those kernels wrote, and nothing they read that this one writes, may be touched before
+// it.  The second call lets the next kernel's blocks move in as this kernel's leave.  It comes
+// after the wait, so that at most two kernels overlap, and never before a wait for another rank
+// or stream: blocks that are already resident could then take the room that the awaited kernel
+// needs.
+__device__ __forceinline__ void wait_for_previous_kernels() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void let_next_kernel_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 }  // namespace ptx
 }  // namespace pplx

@@ -496,6 +496,7 @@ template <typename T, typename U, bool SEND, bool RECV, bool kLines>
 __global__ void __launch_bounds__(kCombineThreads, 1)
     combine_kernel(const __grid_constant__ CombineArgs a) {
   extern __shared__ __align__(16) uint32_t dyn_smem[];
+  ptx::wait_for_previous_kernels();
   combine_body<T, U, SEND, RECV, kLines>(a, dyn_smem);
 }
 
@@ -525,6 +526,8 @@ cudaError_t launch_typed(const CombineArgs& a, bool send, bool recv, int grid, s
   const void* fn = a.ll ? combine_fn<T, U, true, false>(send, recv)
                         : combine_fn<T, U, false, false>(send, recv);
   void* params[] = {const_cast<CombineArgs*>(&a)};
+  if (a.p.world == 1)
+    return launch_after_previous(fn, dim3(grid), dim3(kCombineThreads), params, smem, stream);
   return cudaLaunchKernel(fn, dim3(grid), dim3(kCombineThreads), params, smem, stream);
 }
 

@@ -222,7 +222,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       (kFromStaging && g.src_table != 0) ? a_row0 + g.num_experts : nullptr;
   const A2AParams& p = g.a2a;
   int parity = 0;
-  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile uint32_t* abort_flag = &ctl->abort_flag;
@@ -249,6 +248,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc::tmem_alloc(&ctl->tmem_base, kTmemCols);
     tc::tmem_relinquish();
   }
+  ptx::wait_for_previous_kernels();
+  if constexpr (!kFromStaging) ptx::let_next_kernel_start();
+  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
   if constexpr (kFromStaging) {
     // Role of the dispatch receive phase: rows per (source, expert) from the posted
     // histograms, the layout of the packed staging, the per-expert totals.
@@ -368,6 +370,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
+      // (The scales' warp waits for the same rows, which have all landed.)
+      if constexpr (kFromStaging) ptx::let_next_kernel_start();
       if (!ok || *abort_flag != 0u) {
         const uint64_t t0 = ptx::globaltimer_ns();
         for (uint32_t s = 0; s < stages; ++s) {

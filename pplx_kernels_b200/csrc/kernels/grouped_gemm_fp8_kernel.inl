@@ -73,7 +73,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       (reinterpret_cast<uintptr_t>(a_row0 + g.num_experts) + 15) & ~static_cast<uintptr_t>(15));
   const A2AParams& p = g.a2a;
   int parity = 0;
-  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile uint32_t* abort_flag = &ctl->abort_flag;
@@ -82,6 +81,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int num_kb = ceil_div<int>(g.k, kBlockKBytes);
 
   if (tid == 0) ctl->abort_flag = 0;
+  ptx::wait_for_previous_kernels();
+  if constexpr (!kFromStaging) ptx::let_next_kernel_start();
+  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
   if constexpr (kFromStaging) {
     // Role of the dispatch receive phase: rows per (source, expert) from the posted
     // histograms, the layout of the packed staging, the per-expert totals.

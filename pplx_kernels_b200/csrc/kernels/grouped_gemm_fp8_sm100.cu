@@ -235,8 +235,10 @@ void launch_fp8(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b, const Fp8G
   CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
   const int grid = num_sms > 0 ? num_sms : get_sm_count();
-  kernel<<<grid, kThreads, smem, stream>>>(tmap_a, tmap_b, g);
-  CUDA_CHECK(cudaGetLastError());
+  void* params[] = {const_cast<CUtensorMap*>(&tmap_a), const_cast<CUtensorMap*>(&tmap_b),
+                    const_cast<Fp8GemmArgs*>(&g)};
+  CUDA_CHECK(launch_after_previous(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(kThreads),
+                                   params, smem, stream));
 }
 
 // Token rows come in boxes of 64 and 16.
@@ -266,8 +268,10 @@ void launch_fold(const CUtensorMap& tmap_w, const TokenMaps& x, Fp8GemmArgs g, i
   CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
   const int grid = num_sms > 0 ? num_sms : get_sm_count();
-  kernel<<<grid, kThreads, smem, stream>>>(tmap_w, x.x64, x.x16, g);
-  CUDA_CHECK(cudaGetLastError());
+  void* params[] = {const_cast<CUtensorMap*>(&tmap_w), const_cast<CUtensorMap*>(&x.x64),
+                    const_cast<CUtensorMap*>(&x.x16), &g};
+  CUDA_CHECK(launch_after_previous(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(kThreads),
+                                   params, smem, stream));
 }
 
 }  // namespace

@@ -188,7 +188,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* src_rows = (kFromStaging && g.src_table != 0) ? x_row0 + g.num_experts : nullptr;
   const A2AParams& p = g.a2a;
   int parity = 0;
-  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
 
   const uint32_t cta_rank = kPair ? tc::cluster_ctarank() : 0u;
   const bool leader = cta_rank == 0u;
@@ -227,6 +226,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       tc::tmem_relinquish();
     }
   }
+  ptx::wait_for_previous_kernels();
+  if constexpr (!kFromStaging) ptx::let_next_kernel_start();
+  if constexpr (kFromStaging || kToPeers) parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
   if constexpr (kFromStaging) {
     // Role of the dispatch receive phase: learn how many rows every source sends
     // to every local expert, lay the rows out, publish the per-expert totals.
@@ -388,6 +390,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
+      // (Nothing is waited for any more that another stream or rank has to do.)
+      if constexpr (kFromStaging) ptx::let_next_kernel_start();
       if (!ok || *abort_flag != 0u) {
         // Give the loads already issued a bounded time to land before the CTA
         // leaves: their destination is this CTA's shared memory.
@@ -712,19 +716,10 @@ void launch_one(const CUtensorMap& tmap_w, const TokenMaps& tmap_x, GroupedGemmA
   const size_t smem = fixed + g.ring_bytes;
   CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(kPair ? (grid & ~1) : grid);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = kPair ? 2 : 1;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, tmap_w, tmap_x, g));
+  void* params[] = {const_cast<CUtensorMap*>(&tmap_w), const_cast<TokenMaps*>(&tmap_x), &g};
+  CUDA_CHECK(launch_after_previous(reinterpret_cast<const void*>(kernel),
+                                   dim3(kPair ? (grid & ~1) : grid), dim3(kThreads), params, smem,
+                                   stream, kPair ? 2 : 1));
 }
 
 template <bool SWIGLU, bool kFromStaging, bool kToPeers>

@@ -133,6 +133,8 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
   const int E = p.num_experts, topk = p.topk;
   const int entries = entry_cap(p);
   const Smem sm = carve(dyn_smem, entries, E);
+  ptx::wait_for_previous_kernels();
+  ptx::let_next_kernel_start();
   stamp(p, kTrDispatchStart, kTrDispatchStart);
   stamp_block(p, kTrBlockDispatchStart);
 
@@ -391,6 +393,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
     single_unstage_kernel(const __grid_constant__ DispatchArgs a, int chunks_sent) {
   __shared__ uint32_t s_tokens;
   const A2AParams& p = a.p;
+  ptx::wait_for_previous_kernels();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int topk = p.topk;
   const int nvec = p.hidden_bytes >> 4;
@@ -457,6 +460,8 @@ template <typename T, typename U, int kVec>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
     single_combine_kernel(const __grid_constant__ CombineArgs a) {
   const A2AParams& p = a.p;
+  ptx::wait_for_previous_kernels();
+  ptx::let_next_kernel_start();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m = token_count(a.bound_m, a.num_tokens, p.max_tokens);
   const int topk = p.topk;
@@ -566,7 +571,7 @@ cudaError_t launch(const void* fn, int grid, size_t smem, void** params, cudaStr
                                                  static_cast<int>(smem));
     if (err != cudaSuccess) return err;
   }
-  return cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), params, smem, stream);
+  return launch_after_previous(fn, dim3(grid), dim3(kThreads), params, smem, stream);
 }
 
 }  // namespace
