@@ -8,32 +8,24 @@
 // (the DeepSeek-V3 / Qwen3 fp8 checkpoint format).  The reference has no GEMM;
 // this kernel is the fp8 arm of the MoE layer that goes beyond it.
 //
-// fp32 scales per 128 columns are not the hardware's block-scale format, so each
-// 128-wide K block is multiplied on the tensor cores into one of two scratch
-// accumulators in tensor memory (four K = 32 MMAs, M = 128, N = 256) and eight
-// epilogue warps fold it, times the two scales, into the running result that
-// they keep in REGISTERS: warps 4-7 own output columns [0, 64) of each half of the
-// tile, warps 8-11 columns [64, 128), so a thread holds 128 fp32 accumulators and
-// only reads tensor memory (tcgen05.ld), while the MMAs of the next K block fill
-// the other scratch accumulator.
+// Two kernels: grouped_gemm_fp8_fold.inl for arbitrary fp32 scales, which the CUDA cores apply per
+// 128-wide K block, and grouped_gemm_fp8_mx.inl for power-of-two scales (`pow2_scales`), which the
+// tensor cores apply.  In both the weights are the M operand and the tokens the N operand.
 //
-// With power-of-two scales (`pow2_scales`) the tensor cores apply them themselves
-// (kind::mxf8f6f4.block_scale): warp 3 turns the fp32 scales of each K block into E8M0 bytes in
-// the layout tcgen05.cp takes, the MMA thread copies them into tensor memory in front of the
-// block's four MMAs, the whole K range accumulates in ONE tensor-memory accumulator, and the
-// fold warps only read the finished tile (and free the accumulator before they convert and
-// store, so that the next tile's MMAs run under the epilogue).
-//
-// Epilogues:  kBf16   plain down projection, bf16 result, 256 columns per tile
+// Epilogues:  plain   down projection, bf16 result
 //             kSwiGLUQuant   w stacks gate and up rows; the tile is 128 gate + 128 up
 //                     rows, the result silu(gate) * up is 128 columns = exactly one
-//                     scale block, so it is quantised right here to e4m3 + one fp32
+//                     scale block, so it is quantised right here to e4m3 + one
 //                     scale per row and tile -- the input format of the next GEMM.
 //
-// Roles: warp 0 TMA producer, warp 1 MMA issuer, warp 2 tensor-memory allocation,
-// warps 4-11 scale-and-accumulate + epilogue.  All waits are bounded; on expiry the
-// CTA drains, frees its tensor memory and reports through *status.
+// kFromStaging: the tokens and their scales are read out of the dispatch staging arena that
+// peers fill (packed, quantising send); tiles wait for the sources they cover.
+// kToPeers: the bf16 result rows go to the combine staging of the tokens' home ranks.
+//
+// All waits are bounded; on expiry the CTA drains, frees its tensor memory and reports through
+// *status.
 #include <algorithm>
+#include <type_traits>
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -53,85 +45,39 @@ namespace pplx {
 namespace {
 
 constexpr int kBlockM = 128;
-constexpr int kTileN = 256;        // weight rows per tile (UMMA N)
 constexpr int kBlockKBytes = 128;  // 128 e4m3 values = one swizzle row = one scale block
 constexpr int kUmmaKBytes = 32;
-constexpr int kStages = 4;
 constexpr int kThreads = 384;
-constexpr int kTmemCols = 512;     // two scratch accumulators of 256 columns
-constexpr uint32_t kABytes = kBlockM * kBlockKBytes;
-constexpr uint32_t kBBytes = kTileN * kBlockKBytes;
-constexpr uint32_t kStageBytes = kABytes + kBBytes;
-constexpr uint32_t kSfAtomBytes = 512;
-constexpr uint32_t kSfStageBytes = 3 * kSfAtomBytes;
-constexpr uint32_t kSfaCol = 256;  // tensor-memory columns of the scales, behind the accumulator
-constexpr uint32_t kSfbCol = 260;
+constexpr int kTmemCols = 512;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 constexpr int kMaxExperts = 1024;
 
-struct SharedControl {
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
-  uint64_t part_full[2];   // scratch accumulator holds a finished K block
-  uint64_t part_empty[2];  // scratch accumulator may be overwritten
-  uint64_t acc_full;       // hardware-scaled form: the tile's accumulator is complete
-  uint64_t acc_empty;      //                       ... has been read out by all fold warps
-  uint32_t tmem_base;
-  uint32_t abort_flag;
-  float row_amax[2][kBlockM];  // SwiGLU epilogue: per-row maxima of the two column halves
-  uint32_t sig_token[kBlockM];  // peer-storing epilogue: token of each tile row
-  uint32_t sig_group[kBlockM];  //                        first rank of the token's DP group
-  // Hardware-scaled form: per stage the E8M0 scales of the K block in the layout tcgen05.cp
-  // takes (32 rows of 16 bytes per 128 rows or columns): A rows, B columns 0-127, 128-255.
-  alignas(128) uint8_t sf[kStages][kSfStageBytes];
-};
-
-constexpr uint32_t kNoSignalFp8 = 0xffffffffu;
-
-// Staging of the peer-storing epilogue: per fold warp 32 rows x (64 B + 16 B pad).
-constexpr int kFp8StageRowBytes = 80;
-constexpr uint32_t kSignalQueue = 512;
-struct Fp8PeerStage {
-  uint8_t rows[8][32][kFp8StageRowBytes];
-  unsigned long long row_off[kBlockM];  // arena offset of each tile row's combine slot
-  uint32_t q_token[kSignalQueue];        // queued arrival adds: token ...
-  uint32_t q_group_units[kSignalQueue];  // ... first rank of its DP group | columns << 8
-};
-
 __device__ __forceinline__ float silu(float v) { return v / (1.0f + __expf(-v)); }
 
-// 32 lanes x 16 consecutive columns.
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-
-struct Fp8Tile {
-  int expert, m_blk, n_blk, rows;
+struct Fp8GemmArgs {
+  const int32_t* counts;   // [E]
+  const float* sa;         // [E][rows][kblocks]
+  int64_t sa_stride_e, sa_stride_row;
+  const float* sw;         // [E][ceil(w_rows / 128)][kblocks]
+  int64_t sw_stride_e, sw_stride_row;
+  void* out;               // bf16 [E][rows][n_out]  or  e4m3 [E][rows][n_out]
+  int64_t out_stride_e, out_stride_row;  // elements
+  float* out_scale;        // kSwiGLUQuant: [E][rows][n_out / 128]
+  int64_t os_stride_e, os_stride_row;
+  uint32_t* status;
+  int num_experts, rows_per_expert, n_out, k;
+  // Only read by the forms fused with the all-to-all:
+  int32_t* out_num_tokens;  // optional [nle]: per-expert totals for the caller
+  int src_table;            // keep rows per (expert, source) in shared memory
+  uint32_t ring_bytes;      // shared memory for the stages (set by the launcher)
+  A2AParams a2a;
 };
-
-__device__ __forceinline__ Fp8Tile locate(const uint32_t* tile_start, const uint32_t* rows_of,
-                                          int num_experts, uint32_t t) {
-  Fp8Tile c;
-  c.expert = find_group(tile_start, num_experts, t);
-  c.rows = static_cast<int>(rows_of[c.expert]);
-  const int m_tiles = ceil_div<int>(c.rows, kBlockM);
-  const uint32_t rem = t - tile_start[c.expert];
-  c.n_blk = static_cast<int>(rem / m_tiles);
-  c.m_blk = static_cast<int>(rem - static_cast<uint32_t>(c.n_blk) * m_tiles);
-  return c;
-}
 
 }  // namespace
 }  // namespace pplx
 
-#include "grouped_gemm_fp8_kernel.inl"
 #include "grouped_gemm_fp8_fold.inl"
+#include "grouped_gemm_fp8_mx.inl"
 
 namespace pplx {
 namespace {
@@ -181,12 +127,6 @@ namespace {
 
 constexpr size_t kMaxSrcEntriesFp8 = 2048;
 
-size_t fp8_smem_bytes(size_t experts, size_t src_entries, bool to_peers) {
-  return 1024 + kStages * kStageBytes + sizeof(SharedControl) +
-         sizeof(uint32_t) * (3 * experts + 1 + src_entries) +
-         (to_peers ? sizeof(Fp8PeerStage) + 16 : 0);
-}
-
 void check_fp8_call(const Fp8GemmCall& c, bool need_x, bool need_out) {
   PPLX_CHECK(c.num_experts > 0 && c.num_experts <= kMaxExperts, "num_experts out of range");
   PPLX_CHECK(c.k > 0 && c.k % 16 == 0, "K must be a positive multiple of 16");
@@ -223,24 +163,6 @@ Fp8GemmArgs fp8_args(const Fp8GemmCall& c) {
   return g;
 }
 
-template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers, bool kPow2 = false>
-void launch_fp8(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b, const Fp8GemmArgs& g,
-                int num_sms, cudaStream_t stream) {
-  auto* kernel = grouped_gemm_fp8_kernel<kSwiGLUQuant, kFromStaging, kToPeers, kPow2>;
-  const size_t src_entries =
-      (kFromStaging && g.src_table != 0) ? static_cast<size_t>(g.num_experts) * g.a2a.world : 0;
-  const size_t smem = fp8_smem_bytes(g.num_experts, src_entries, kToPeers);
-  PPLX_CHECK(smem <= 227 * 1024, "the tile tables of " << g.num_experts << " experts need "
-                                                       << smem << " bytes of shared memory");
-  CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
-  const int grid = num_sms > 0 ? num_sms : get_sm_count();
-  void* params[] = {const_cast<CUtensorMap*>(&tmap_a), const_cast<CUtensorMap*>(&tmap_b),
-                    const_cast<Fp8GemmArgs*>(&g)};
-  CUDA_CHECK(launch_after_previous(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(kThreads),
-                                   params, smem, stream));
-}
-
 // Token rows come in boxes of 64 and 16.
 struct TokenMaps {
   CUtensorMap x64, x16;
@@ -252,17 +174,29 @@ TokenMaps make_token_maps(const void* base, int64_t planes, int64_t rows, int64_
           make_byte_map(base, planes, rows, k, stride_row, stride_plane, 16)};
 }
 
-template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers>
-void launch_fold(const CUtensorMap& tmap_w, const TokenMaps& x, Fp8GemmArgs g, int num_sms,
+// `kPow2`: the form whose scales the tensor cores apply.
+template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers, bool kPow2>
+void launch_form(const CUtensorMap& tmap_w, const TokenMaps& x, Fp8GemmArgs g, int num_sms,
                  cudaStream_t stream) {
-  auto* kernel = fold::grouped_gemm_fp8_fold_kernel<kSwiGLUQuant, kFromStaging, kToPeers>;
+  using Control = std::conditional_t<kPow2, mx::Control, fold::Control>;
+  const void* kernel;
+  if constexpr (kPow2)
+    kernel = reinterpret_cast<const void*>(
+        &mx::grouped_gemm_fp8_mx_kernel<kSwiGLUQuant, kFromStaging, kToPeers>);
+  else
+    kernel = reinterpret_cast<const void*>(
+        &fold::grouped_gemm_fp8_fold_kernel<kSwiGLUQuant, kFromStaging, kToPeers>);
   const size_t src_entries =
       (kFromStaging && g.src_table != 0) ? static_cast<size_t>(g.num_experts) * g.a2a.world : 0;
-  const size_t fixed = 1024 + sizeof(fold::Control) + (kToPeers ? sizeof(tok::PeerStage) : 0) +
+  const size_t fixed = 1024 + sizeof(Control) + (kToPeers ? sizeof(tok::PeerStage) : 0) +
                        sizeof(uint32_t) * (3 * static_cast<size_t>(g.num_experts) + 1 + src_entries);
-  // The stages take what the tables leave: four of the widest tiles fit beside any table the
-  // checks admit.
+  // The stages take what the tables leave: at least two of the widest tiles beside any table the
+  // checks admit, three beside those of 256 experts.
   constexpr size_t kSmem = 227 * 1024;
+  static_assert(kSmem - (1024 + sizeof(Control) + sizeof(tok::PeerStage) +
+                         sizeof(uint32_t) * (3 * kMaxExperts + 1 + kMaxSrcEntriesFp8)) >=
+                    2 * (mx::kWBytes + mx::kMaxTokens * kBlockKBytes) + 1024,
+                "too little shared memory for the stages");
   g.ring_bytes = static_cast<uint32_t>((kSmem - fixed) & ~static_cast<size_t>(1023));
   const size_t smem = fixed + g.ring_bytes;
   CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -270,29 +204,28 @@ void launch_fold(const CUtensorMap& tmap_w, const TokenMaps& x, Fp8GemmArgs g, i
   const int grid = num_sms > 0 ? num_sms : get_sm_count();
   void* params[] = {const_cast<CUtensorMap*>(&tmap_w), const_cast<CUtensorMap*>(&x.x64),
                     const_cast<CUtensorMap*>(&x.x16), &g};
-  CUDA_CHECK(launch_after_previous(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(kThreads),
-                                   params, smem, stream));
+  CUDA_CHECK(launch_after_previous(kernel, dim3(grid), dim3(kThreads), params, smem, stream));
+}
+
+template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers>
+void launch_fp8(const Fp8GemmCall& c, const TokenMaps& x, const Fp8GemmArgs& g, cudaStream_t stream) {
+  const int64_t w_rows = (kSwiGLUQuant ? 2 : 1) * static_cast<int64_t>(c.n_out);
+  const CUtensorMap tmap_w =
+      make_byte_map(c.w, c.num_experts, w_rows, c.k, c.w_stride_row, c.w_stride_e);
+  if (c.pow2_scales)
+    launch_form<kSwiGLUQuant, kFromStaging, kToPeers, true>(tmap_w, x, g, c.num_sms, stream);
+  else
+    launch_form<kSwiGLUQuant, kFromStaging, kToPeers, false>(tmap_w, x, g, c.num_sms, stream);
 }
 
 }  // namespace
 
 void launch_grouped_gemm_fp8(const Fp8GemmCall& c, cudaStream_t stream) {
   check_fp8_call(c, true, true);
-  const int64_t w_rows = c.swiglu_quant ? 2 * static_cast<int64_t>(c.n_out) : c.n_out;
-  const CUtensorMap tmap_a =
-      make_byte_map(c.x, c.num_experts, c.rows_per_expert, c.k, c.x_stride_row, c.x_stride_e);
-  const CUtensorMap tmap_b =
-      make_byte_map(c.w, c.num_experts, w_rows, c.k, c.w_stride_row, c.w_stride_e);
-  const Fp8GemmArgs g = fp8_args(c);
-  if (c.pow2_scales) {
-    if (c.swiglu_quant) launch_fp8<true, false, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
-    else launch_fp8<false, false, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
-    return;
-  }
   const TokenMaps x = make_token_maps(c.x, c.num_experts, c.rows_per_expert, c.k, c.x_stride_row,
                                       c.x_stride_e);
-  if (c.swiglu_quant) launch_fold<true, false, false>(tmap_b, x, g, c.num_sms, stream);
-  else launch_fold<false, false, false>(tmap_b, x, g, c.num_sms, stream);
+  if (c.swiglu_quant) launch_fp8<true, false, false>(c, x, fp8_args(c), stream);
+  else launch_fp8<false, false, false>(c, x, fp8_args(c), stream);
 }
 
 void launch_gemm_fp8_from_staging(const Fp8GemmCall& c, const A2AParams& p,
@@ -304,23 +237,15 @@ void launch_gemm_fp8_from_staging(const Fp8GemmCall& c, const A2AParams& p,
              "fp32 scale per 128 columns");
   PPLX_CHECK(c.k == p.hidden_dim && c.num_experts == p.nle && c.rows_per_expert >= p.cap,
              "shape mismatch between the GEMM and the all-to-all");
-  // A: [1][world * region_slots][hidden] e4m3 view of this rank's packed staging.
+  // Tokens: [1][world * region_slots][hidden] e4m3 view of this rank's packed staging.
   const int64_t slots = static_cast<int64_t>(p.world) * p.region_slots;
-  const CUtensorMap tmap_a = make_byte_map(p.peer[p.rank] + p.off_disp_stage, 1, slots,
-                                           p.hidden_dim, p.slot_bytes, slots * p.slot_bytes);
-  const CUtensorMap tmap_b = make_byte_map(c.w, c.num_experts, 2 * static_cast<int64_t>(c.n_out),
-                                           c.k, c.w_stride_row, c.w_stride_e);
+  const TokenMaps x = make_token_maps(p.peer[p.rank] + p.off_disp_stage, 1, slots, p.hidden_dim,
+                                      p.slot_bytes, slots * p.slot_bytes);
   Fp8GemmArgs g = fp8_args(c);
   g.out_num_tokens = out_num_tokens;
   g.a2a = p;
   g.src_table = static_cast<size_t>(p.nle) * p.world <= kMaxSrcEntriesFp8 ? 1 : 0;
-  if (c.pow2_scales) {
-    launch_fp8<true, true, false, true>(tmap_a, tmap_b, g, c.num_sms, stream);
-    return;
-  }
-  const TokenMaps x = make_token_maps(p.peer[p.rank] + p.off_disp_stage, 1, slots, p.hidden_dim,
-                                      p.slot_bytes, slots * p.slot_bytes);
-  launch_fold<true, true, false>(tmap_b, x, g, c.num_sms, stream);
+  launch_fp8<true, true, false>(c, x, g, stream);
 }
 
 void launch_gemm_fp8_to_peers(const Fp8GemmCall& c, const A2AParams& p, cudaStream_t stream) {
@@ -331,20 +256,12 @@ void launch_gemm_fp8_to_peers(const Fp8GemmCall& c, const A2AParams& p, cudaStre
   PPLX_CHECK(c.counts == reinterpret_cast<const int32_t*>(p.recv_count),
              "counts must be the all-to-all's received-row counts");
   PPLX_CHECK(p.dp_size <= 8, "at most 8 replicas per DP group");
-  const CUtensorMap tmap_a =
-      make_byte_map(c.x, c.num_experts, c.rows_per_expert, c.k, c.x_stride_row, c.x_stride_e);
-  const CUtensorMap tmap_b =
-      make_byte_map(c.w, c.num_experts, c.n_out, c.k, c.w_stride_row, c.w_stride_e);
+  const TokenMaps x = make_token_maps(c.x, c.num_experts, c.rows_per_expert, c.k, c.x_stride_row,
+                                      c.x_stride_e);
   Fp8GemmArgs g = fp8_args(c);
   g.out = nullptr;
   g.a2a = p;
-  if (c.pow2_scales) {
-    launch_fp8<false, false, true, true>(tmap_a, tmap_b, g, c.num_sms, stream);
-    return;
-  }
-  const TokenMaps x = make_token_maps(c.x, c.num_experts, c.rows_per_expert, c.k, c.x_stride_row,
-                                      c.x_stride_e);
-  launch_fold<false, false, true>(tmap_b, x, g, c.num_sms, stream);
+  launch_fp8<false, false, true>(c, x, g, stream);
 }
 
 }  // namespace pplx
