@@ -53,7 +53,7 @@ struct GroupedGemmCall {
   int num_sms = 0;           // 0 = all
   int half_n = 0;            // 0 = choose; else half of the most token rows per tile, which are
                              // the accumulator's columns (multiple of 8, 16..128)
-  int64_t expected_total_rows = 0;  // kept for callers; the device reads the real counts
+  int64_t expected_total_rows = 0;  // hint for the choice of the kernel form; 0 = capacity
   int cta_pair = -1;         // 0 = one CTA per tile of 128 weight rows, else a CTA pair per
                              // 256 weight rows (tcgen05 cta_group::2) where the grid has two CTAs
 };

@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   Control* ctl = reinterpret_cast<Control*>(ring + g.ring_bytes);
   // (kToPeers only) behind the control block; the tables come last.
-  PeerStage* peer_stage = reinterpret_cast<PeerStage*>(ctl + 1);
+  using Peers = PeerStage<kPeerTokens>;
+  Peers* peer_stage = reinterpret_cast<Peers*>(ctl + 1);
   uint32_t* tile_start = kToPeers ? reinterpret_cast<uint32_t*>(peer_stage + 1)
                                   : reinterpret_cast<uint32_t*>(ctl + 1);  // [E + 1]
   uint32_t* rows_of = tile_start + g.num_experts + 1;                      // [E] valid rows

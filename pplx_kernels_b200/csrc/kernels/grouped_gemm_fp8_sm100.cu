@@ -49,6 +49,7 @@ constexpr int kBlockKBytes = 128;  // 128 e4m3 values = one swizzle row = one sc
 constexpr int kUmmaKBytes = 32;
 constexpr int kThreads = 384;
 constexpr int kTmemCols = 512;
+constexpr int kPeerTokens = 256;   // at least the widest token tile
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 constexpr int kMaxExperts = 1024;
 
@@ -188,12 +189,12 @@ void launch_form(const CUtensorMap& tmap_w, const TokenMaps& x, Fp8GemmArgs g, i
         &fold::grouped_gemm_fp8_fold_kernel<kSwiGLUQuant, kFromStaging, kToPeers>);
   const size_t src_entries =
       (kFromStaging && g.src_table != 0) ? static_cast<size_t>(g.num_experts) * g.a2a.world : 0;
-  const size_t fixed = 1024 + sizeof(Control) + (kToPeers ? sizeof(tok::PeerStage) : 0) +
+  const size_t fixed = 1024 + sizeof(Control) + (kToPeers ? sizeof(tok::PeerStage<kPeerTokens>) : 0) +
                        sizeof(uint32_t) * (3 * static_cast<size_t>(g.num_experts) + 1 + src_entries);
   // The stages take what the tables leave: at least two of the widest tiles beside any table the
   // checks admit, three beside those of 256 experts.
   constexpr size_t kSmem = 227 * 1024;
-  static_assert(kSmem - (1024 + sizeof(Control) + sizeof(tok::PeerStage) +
+  static_assert(kSmem - (1024 + sizeof(Control) + sizeof(tok::PeerStage<kPeerTokens>) +
                          sizeof(uint32_t) * (3 * kMaxExperts + 1 + kMaxSrcEntriesFp8)) >=
                     2 * (mx::kWBytes + mx::kMaxTokens * kBlockKBytes) + 1024,
                 "too little shared memory for the stages");

@@ -9,10 +9,11 @@
 //
 // The WEIGHTS are the M operand of the MMAs and the tokens the N operand.  A CTA pair
 // (tcgen05 cta_group::2) owns a tile of 256 weight rows, 128 in each CTA's tensor-memory
-// lanes, times a token tile of 32 to 256 rows of one expert in steps of 32; each CTA loads its
+// lanes, times a token tile of 32 to 512 rows of one expert in steps of 32; each CTA loads its
 // own weight rows and HALF of the tokens, and the leader's MMAs read both CTAs' shared
 // memory.  An expert's rows are cut into equal token tiles (to a step), so
-//   - weights cross from DRAM once and from L2 once for up to 256 rows of an expert,
+//   - weights cross from DRAM once and from L2 once for up to 512 rows of an expert (two MMAs per
+//     step above 256),
 //   - the work follows the rows there are, to a multiple of 32: with the tokens as M every
 //     expert was padded to a multiple of 128 rows (256 for pairs, which therefore were only
 //     used from 2048 rows per expert on),
@@ -28,7 +29,7 @@
 //
 // Roles (persistent over tiles): warp 0 TMA producer, warp 1 MMA issuer (leader CTA only),
 // warp 2 tensor-memory allocation, warps 4-11 epilogue.  Two accumulators of 256 columns let
-// the epilogue of a tile run under the MMAs of the next.  No TMA multicast is involved: the two
+// the epilogue of a tile run under the MMAs of the next; wider tiles have one of 512 columns.  No TMA multicast is involved: the two
 // CTAs load different data; only barrier arrivals (tcgen05.commit) are delivered to both.
 //
 // Tiles are (expert, block of weight rows, token tile) with the token tile varying fastest, so
@@ -77,17 +78,19 @@ namespace {
 using namespace tok;
 
 constexpr int kBlockM = 128;      // weight rows per CTA and tile
-constexpr int kMaxTokens = 256;   // token rows per tile
+constexpr int kMmaTokens = 256;   // token rows per MMA
+constexpr int kMaxTokens = 512;   // token rows per tile
 constexpr int kBlockK = 64;       // 64 bf16 = one 128-byte swizzle row
 constexpr int kUmmaK = 16;
 constexpr int kMaxStages = 12;
 constexpr int kThreads = 384;
-constexpr int kTmemCols = 512;    // two accumulators of kMaxTokens columns
+constexpr int kTmemCols = 512;    // an accumulator of kMaxTokens columns, or two of half of them
 constexpr uint32_t kRowBytes = kBlockK * 2;
 constexpr uint32_t kWBytes = kBlockM * kRowBytes;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s per wait
 constexpr int kMaxExperts = 1024;
-constexpr int kTileOverhead = 16;     // ... of a tile, in token rows
+constexpr int kDrainPlain = 8;    // cycles per token row to read out an accumulator that is the only
+constexpr int kDrainSwiglu = 35;  // one, as fitted to the times of both widths at 512 rows
 constexpr int kSegBytes = 256 + 16;  // 128 bf16 columns of one token, padded
 
 struct Control {
@@ -158,6 +161,11 @@ __device__ __forceinline__ uint32_t swiglu_pair(uint32_t g0, uint32_t g1, uint32
                    silu(__uint_as_float(g1)) * __uint_as_float(u1));
 }
 
+// Token rows of a tile that its first MMA takes; the second takes the rest.
+__device__ __forceinline__ int first_mma(int width) {
+  return width <= kMmaTokens ? width : ((width >> 1) + 31) & ~31;
+}
+
 template <bool kPair>
 __device__ __forceinline__ void load_rows(void* dst, const CUtensorMap* map, uint64_t* full, int k,
                                           int row, int plane) {
@@ -165,11 +173,12 @@ __device__ __forceinline__ void load_rows(void* dst, const CUtensorMap* map, uin
   else tc::tma_load_3d(dst, map, full, k, row, plane);
 }
 
-template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kPair>
+template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kPair, bool kWide>
 __global__ void __launch_bounds__(kThreads, 1)
     grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                         const __grid_constant__ TokenMaps tmap_x,
                         const __grid_constant__ GroupedGemmArgs g) {
+  static_assert(kPair || !kWide, "one CTA has no room for the stages of wide tiles");
   constexpr int kCtas = kPair ? 2 : 1;
   constexpr int kUnit = 16 * kCtas;  // steps of an MMA's N: 16, or 32 for M = 256 over a pair
   constexpr int kCols = SWIGLU ? kBlockM / 2 : kBlockM;  // output columns per CTA and tile
@@ -178,7 +187,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   Control* ctl = reinterpret_cast<Control*>(ring + g.ring_bytes);
   // (kToPeers only) behind the control block; the tables come last.
-  PeerStage* peer_stage = reinterpret_cast<PeerStage*>(ctl + 1);
+  using Peers = PeerStage<kWide ? kMaxTokens : kMmaTokens>;
+  Peers* peer_stage = reinterpret_cast<Peers*>(ctl + 1);
   uint32_t* tile_start = kToPeers ? reinterpret_cast<uint32_t*>(peer_stage + 1)
                                   : reinterpret_cast<uint32_t*>(ctl + 1);  // [E + 1]
   uint32_t* rows_of = tile_start + g.num_experts + 1;                      // [E] valid rows
@@ -289,14 +299,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   __syncthreads();
 
-  // The most token rows a tile may have.  One tile per expert where that is possible: below
-  // 256 rows an expert is bound by its weights, which more tiles would only read again.  Above,
-  // the limit that minimises (waves of tiles) x (time of a tile); the time of a tile is its
-  // width plus a constant for its barriers and its share of the epilogue.  Every CTA computes
-  // the same.
-  int limit = g.max_tokens / kUnit * kUnit;
-  if (ctl->max_rows > static_cast<uint32_t>(limit)) {
-    for (int cand = limit - kUnit * warp; 2 * cand >= limit; cand -= kUnit * (kThreads / 32)) {
+  // The most token rows a tile may have.  One tile per expert up to 256 rows: there an expert is
+  // bound by its weights, which more tiles would only read again.  Above, the limit that
+  // minimises (waves of tiles) x (time of a tile).  Per K block of 64 a tile of w rows takes 2 * w
+  // cycles of MMAs, or as long as L2 needs for 16 KB of weights and 64 * w bytes of tokens per CTA
+  // at 64 bytes per cycle; more than 256 rows leave no second accumulator, so their epilogue is
+  // not hidden.  Every CTA computes the same.
+  constexpr uint32_t kDrain = SWIGLU ? kDrainSwiglu : kDrainPlain;
+  int limit = min(g.max_tokens, kWide ? kMaxTokens : kMmaTokens) / kUnit * kUnit;
+  if (ctl->max_rows > static_cast<uint32_t>(min(limit, kMmaTokens))) {
+    for (int cand = limit - kUnit * warp; 4 * cand >= limit; cand -= kUnit * (kThreads / 32)) {
       uint32_t tiles = 0, width = 0;
       for (int e = lane; e < g.num_experts; e += 32) {
         const Cut<kUnit> cut(static_cast<int>(rows_of[e]), cand);
@@ -307,12 +319,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       width = __reduce_add_sync(0xffffffffu, width);
       if (lane == 0) {
         const uint64_t waves = ceil_div<uint64_t>(static_cast<uint64_t>(tiles) * w_blocks, workers);
-        const uint64_t cost = waves * (16ull * width / tiles + 16 * kTileOverhead);
-        atomicMin(&ctl->best_limit, (cost << 16) | static_cast<uint64_t>(512 - cand));
+        const uint32_t w = width / tiles;
+        const uint64_t cost = waves * (static_cast<uint64_t>(num_kb) * max(2u * w, 256u + w) +
+                                       (cand > kMmaTokens ? kDrain * w : 0u));
+        atomicMin(&ctl->best_limit, (cost << 16) | static_cast<uint64_t>(kMaxTokens - cand));
       }
     }
     __syncthreads();
-    limit = 512 - static_cast<int>(ctl->best_limit & 0xffffu);
+    limit = kMaxTokens - static_cast<int>(ctl->best_limit & 0xffffu);
   }
   for (int e = tid; e < g.num_experts; e += blockDim.x) {
     const Cut<kUnit> cut(static_cast<int>(rows_of[e]), limit);
@@ -331,6 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // As many stages as the launch's widest token tile leaves room for.
   const uint32_t stage_bytes = kWBytes + ctl->max_width / kCtas * kRowBytes;
   const uint32_t stages = min(g.ring_bytes / stage_bytes, static_cast<uint32_t>(kMaxStages));
+  const bool two = !kWide || ctl->max_width <= kMmaTokens;  // two accumulators
 
   // ---- roles ----------------------------------------------------------------
   if (warp == 0) {
@@ -355,11 +370,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
         }
-        const int own = c.width / kCtas;  // this CTA's share of the tokens
-        const int x_row = static_cast<int>(x_row0[c.expert]) + c.first + static_cast<int>(cta_rank) * own;
+        // This CTA's share of the tokens of each MMA.
+        const int n0 = kWide ? first_mma(c.width) : c.width;
+        const int own0 = n0 / kCtas, own1 = (c.width - n0) / kCtas;
+        const int row0 = static_cast<int>(x_row0[c.expert]) + c.first + static_cast<int>(cta_rank) * own0;
+        const int row1 = row0 - static_cast<int>(cta_rank) * own0 + n0 + static_cast<int>(cta_rank) * own1;
         const int x_plane = kFromStaging ? 0 : c.expert;
         const int w_row = (c.w_blk * kCtas + static_cast<int>(cta_rank)) * kCols;
-        const uint32_t tx = kCtas * (kWBytes + static_cast<uint32_t>(own) * kRowBytes);
+        const uint32_t tx = kCtas * kWBytes + static_cast<uint32_t>(c.width) * kRowBytes;
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = tc::mbar_wait(&ctl->empty[stage], phase ^ 1u, abort_flag, kWaitLimitNs);
           if (!ok) break;
@@ -380,10 +398,17 @@ __global__ void __launch_bounds__(kThreads, 1)
             load_rows<kPair>(w_dst, &tmap_w, full, kb * kBlockK, w_row, c.expert);
           }
           int r = 0;
-          for (; r + 64 <= own; r += 64)
-            load_rows<kPair>(x_dst + r * kRowBytes, &tmap_x.x64, full, kb * kBlockK, x_row + r, x_plane);
-          for (; r < own; r += 16)
-            load_rows<kPair>(x_dst + r * kRowBytes, &tmap_x.x16, full, kb * kBlockK, x_row + r, x_plane);
+          for (; r + 64 <= own0; r += 64, x_dst += 64 * kRowBytes)
+            load_rows<kPair>(x_dst, &tmap_x.x64, full, kb * kBlockK, row0 + r, x_plane);
+          for (; r < own0; r += 16, x_dst += 16 * kRowBytes)
+            load_rows<kPair>(x_dst, &tmap_x.x16, full, kb * kBlockK, row0 + r, x_plane);
+          if constexpr (kWide) {
+            r = 0;
+            for (; r + 64 <= own1; r += 64, x_dst += 64 * kRowBytes)
+              load_rows<kPair>(x_dst, &tmap_x.x64, full, kb * kBlockK, row1 + r, x_plane);
+            for (; r < own1; r += 16, x_dst += 16 * kRowBytes)
+              load_rows<kPair>(x_dst, &tmap_x.x16, full, kb * kBlockK, row1 + r, x_plane);
+          }
           if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
@@ -413,13 +438,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool ok = *abort_flag == 0u;
       for (uint32_t t = worker; t < total_tiles && ok; t += workers, ++local) {
         const Tile c = locate<kUnit>(tile_start, rows_of, g.num_experts, limit, t);
-        const uint32_t idesc = tc::make_instr_desc(1u, kBlockM * kCtas, c.width);
-        const uint32_t buf = local & 1u;
-        const uint32_t use = local >> 1;  // how often this accumulator was used before
+        const int n0 = kWide ? first_mma(c.width) : c.width, n1 = c.width - n0;
+        const uint32_t idesc = tc::make_instr_desc(1u, kBlockM * kCtas, n0);
+        const uint32_t idesc1 = tc::make_instr_desc(1u, kBlockM * kCtas, n1);
+        const uint32_t buf = two ? local & 1u : 0u;
+        const uint32_t use = two ? local >> 1 : local;  // how often this accumulator was used before
         ok = tc::mbar_wait(&ctl->tmem_empty[buf], (use & 1u) ^ 1u, abort_flag, kWaitLimitNs);
         if (!ok) break;
         tc::tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + buf * kMaxTokens;
+        const uint32_t tmem_d = tmem_base + buf * kMmaTokens;
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = tc::mbar_wait(&ctl->full[stage], phase, abort_flag, kWaitLimitNs);
           if (!ok) break;
@@ -433,6 +460,16 @@ __global__ void __launch_bounds__(kThreads, 1)
             const uint64_t xd = tc::advance_smem_desc(x_desc, k * kUmmaK * 2);
             if constexpr (kPair) tc::mma_f16_ss_2cta(tmem_d, wd, xd, idesc, (kb | k) != 0);
             else tc::mma_f16_ss(tmem_d, wd, xd, idesc, (kb | k) != 0);
+          }
+          if constexpr (kWide) {
+            if (n1 > 0) {
+              const uint64_t x1_desc = tc::advance_smem_desc(x_desc, n0 / kCtas * kRowBytes);
+#pragma unroll
+              for (int k = 0; k < kBlockK / kUmmaK; ++k)
+                tc::mma_f16_ss_2cta(tmem_d + n0, tc::advance_smem_desc(w_desc, k * kUmmaK * 2),
+                                    tc::advance_smem_desc(x1_desc, k * kUmmaK * 2), idesc1,
+                                    (kb | k) != 0);
+            }
           }
           // Stage reusable (in both CTAs of a pair) once these MMAs have read it.
           if constexpr (kPair) tc::mma_commit_2cta(&ctl->empty[stage], 0x3);
@@ -460,8 +497,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = *abort_flag == 0u;
     for (uint32_t t = worker; t < total_tiles && ok; t += workers, ++local) {
       const Tile c = locate<kUnit>(tile_start, rows_of, g.num_experts, limit, t);
-      const uint32_t buf = local & 1u;
-      ok = tc::mbar_wait(&ctl->tmem_full[buf], (local >> 1) & 1u, abort_flag, kWaitLimitNs);
+      const uint32_t buf = two ? local & 1u : 0u;
+      ok = tc::mbar_wait(&ctl->tmem_full[buf], (two ? local >> 1 : local) & 1u, abort_flag, kWaitLimitNs);
       // All eight warps leave together or not at all: the barriers below must never be
       // entered by only some of them.
       {
@@ -485,8 +522,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int col0 = (c.w_blk * kCtas + static_cast<int>(cta_rank)) * kCols;
       if constexpr (kFromStaging) {
         // The first block of columns also records where the rows came from.
-        if (col0 == 0 && n_tid < live) {
-          const int row = c.first + n_tid;
+        for (int n = n_tid; col0 == 0 && n < live; n += 256) {
+          const int row = c.first + n;
           const uint8_t* slot = p.peer[p.rank] + p.off_disp_stage +
                                 (static_cast<size_t>(x_row0[c.expert]) + row) * p.slot_bytes;
           const int4 tr = ptx::ld_cg_v4(slot + p.trailer_off);
@@ -499,11 +536,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       if constexpr (kToPeers) {
         // Where each token's row goes, and whose token it is.  (The barrier above comes after
         // the last use of the previous tile's table.)
-        if (n_tid < c.width) {
+        for (int n = n_tid; n < c.width; n += 256) {
           unsigned long long off = 0;
           uint32_t sig_token = kNoSignal, sig_group = 0;
-          if (n_tid < live) {
-            const uint2 rs = p.row_src[static_cast<size_t>(c.expert) * p.cap + c.first + n_tid];
+          if (n < live) {
+            const uint2 rs = p.row_src[static_cast<size_t>(c.expert) * p.cap + c.first + n];
             const int src_rank = static_cast<int>(rs.x & 0xffffu);
             const uint32_t k = rs.x >> 16;
             const uint32_t token = rs.y;
@@ -518,20 +555,31 @@ __global__ void __launch_bounds__(kThreads, 1)
                              token, p.rank);
             }
           }
-          peer_stage->token[n_tid] = sig_token;
-          peer_stage->group[n_tid] = sig_group;
-          peer_stage->row_off[n_tid] = off;
+          peer_stage->token[n] = sig_token;
+          peer_stage->group[n] = sig_group;
+          peer_stage->row_off[n] = off;
         }
         asm volatile("bar.sync 4, 256;" ::: "memory");
       }
       // A thread's values lie across token rows; each group of 16 tokens passes through shared
-      // memory so that rows leave in 16-byte pieces.
-      const uint32_t t_acc = t_lane + buf * kMaxTokens;
+      // memory so that rows leave in 16-byte pieces.  An accumulator that is the only one is
+      // handed back when its last group is in registers (with two of them that was slower).
+      const uint32_t t_acc = t_lane + buf * kMmaTokens;
+      auto hand_back = [&] {
+        tc::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if constexpr (kPair) tc::mbar_arrive_on_leader(&ctl->tmem_empty[buf]);
+          else tc::mbar_arrive(&ctl->tmem_empty[buf]);
+        }
+      };
+      if (kWide && wg >= groups) hand_back();
 #pragma unroll 1
       for (int grp = wg, alt = 0; grp < groups; grp += 2, alt ^= 1) {
         uint32_t lo[8], hi[8];
         load_group(t_acc + grp * 16, lo, hi);
         tc::tmem_ld_wait();
+        if (kWide && grp + 2 >= groups) hand_back();
         uint8_t(*seg)[kSegBytes] = ctl->seg[wg][alt];
         if constexpr (SWIGLU) {
           // Lanes 0-7 of every 16 are gate rows, 8-15 the up rows of the same columns.
@@ -570,13 +618,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      // Accumulator drained: hand it back to the MMA warp.
-      tc::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        if constexpr (kPair) tc::mbar_arrive_on_leader(&ctl->tmem_empty[buf]);
-        else tc::mbar_arrive(&ctl->tmem_empty[buf]);
-      }
+      if constexpr (!kWide) hand_back();
       if constexpr (kToPeers) {
         // Arrival is counted in columns: this tile's share of each row.  The adds are queued
         // and flushed behind ONE system-scope fence for as many tiles as the queue holds.
@@ -697,20 +739,20 @@ TokenMaps make_token_maps(const void* base, int64_t planes, int64_t rows, int64_
 // The per-source table is kept in shared memory when it is at most this many entries.
 constexpr size_t kMaxSrcEntries = 2048;
 
-template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kPair>
+template <bool SWIGLU, bool kFromStaging, bool kToPeers, bool kPair, bool kWide>
 void launch_one(const CUtensorMap& tmap_w, const TokenMaps& tmap_x, GroupedGemmArgs g, int grid,
                 cudaStream_t stream) {
-  auto* kernel = grouped_gemm_kernel<SWIGLU, kFromStaging, kToPeers, kPair>;
+  auto* kernel = grouped_gemm_kernel<SWIGLU, kFromStaging, kToPeers, kPair, kWide>;
   const size_t src_entries =
       (kFromStaging && g.src_table != 0) ? static_cast<size_t>(g.num_experts) * g.a2a.world : 0;
-  const size_t fixed = 1024 + sizeof(Control) + (kToPeers ? sizeof(PeerStage) : 0) +
+  const size_t fixed = 1024 + sizeof(Control) + (kToPeers ? sizeof(PeerStage<kWide ? kMaxTokens : kMmaTokens>) : 0) +
                        sizeof(uint32_t) * (3 * static_cast<size_t>(g.num_experts) + 1 + src_entries);
   // The stages take what the tables leave; kMaxExperts and kMaxSrcEntries leave room for at
-  // least three of the widest tiles.
+  // least three of the widest tiles (four beside the tables of 256 experts).
   constexpr size_t kSmem = 227 * 1024;
-  static_assert(kSmem - (1024 + sizeof(Control) + sizeof(PeerStage) +
+  static_assert(kSmem - (1024 + sizeof(Control) + sizeof(PeerStage<kMaxTokens>) +
                          sizeof(uint32_t) * (3 * kMaxExperts + 1 + kMaxSrcEntries)) >=
-                    3 * (kWBytes + kMaxTokens * kRowBytes) + 1024,
+                    3 * (kWBytes + kMaxTokens / 2 * kRowBytes) + 1024,
                 "too little shared memory for the stages");
   g.ring_bytes = static_cast<uint32_t>((kSmem - fixed) & ~static_cast<size_t>(1023));
   const size_t smem = fixed + g.ring_bytes;
@@ -722,14 +764,29 @@ void launch_one(const CUtensorMap& tmap_w, const TokenMaps& tmap_x, GroupedGemmA
                                    stream, kPair ? 2 : 1));
 }
 
+// Tiles of up to 512 token rows, from an expected mean of 224 rows per expert on: from about there
+// an expert may have more than 256 (and every form takes any number of rows).  8 experts, up /
+// down projection of Mixtral 8x7B, tiles of at most 256 and at most 512 rows: 300 rows each 547 /
+// 276 and 498 / 229 us, 512 rows 750 / 550 and 770 / 383 us, 1024 rows 1370 / 800 and 1410 / 685 us.
+// With few rows, where the weights bound the kernel, it costs 1 to 2 us: 128 rows 325.5 / 169.8
+// and 327.7 / 171.0 us.
+bool want_wide(const GroupedGemmCall& c) {
+  const int64_t rows = c.expected_total_rows > 0
+                           ? c.expected_total_rows
+                           : static_cast<int64_t>(c.num_experts) * c.rows_per_expert;
+  return c.half_n == 0 && rows >= 224 * static_cast<int64_t>(c.num_experts);
+}
+
 template <bool SWIGLU, bool kFromStaging, bool kToPeers>
 void launch_variant(const CUtensorMap& tmap_w, const TokenMaps& tmap_x, const GroupedGemmArgs& g,
                     const GroupedGemmCall& c, cudaStream_t stream) {
   const int grid = c.num_sms > 0 ? c.num_sms : get_sm_count();
-  if (c.cta_pair != 0 && grid >= 2)
-    launch_one<SWIGLU, kFromStaging, kToPeers, true>(tmap_w, tmap_x, g, grid, stream);
+  if (c.cta_pair == 0 || grid < 2)
+    launch_one<SWIGLU, kFromStaging, kToPeers, false, false>(tmap_w, tmap_x, g, grid, stream);
+  else if (want_wide(c))
+    launch_one<SWIGLU, kFromStaging, kToPeers, true, true>(tmap_w, tmap_x, g, grid, stream);
   else
-    launch_one<SWIGLU, kFromStaging, kToPeers, false>(tmap_w, tmap_x, g, grid, stream);
+    launch_one<SWIGLU, kFromStaging, kToPeers, true, false>(tmap_w, tmap_x, g, grid, stream);
 }
 
 void check_common(const GroupedGemmCall& c) {

@@ -17,10 +17,11 @@ namespace tok {
 constexpr uint32_t kNoSignal = 0xffffffffu;
 constexpr int kQueue = 512;  // arrival adds that wait for one fence
 
+template <int kTokens>
 struct PeerStage {
-  unsigned long long row_off[256];      // arena offset of each token's combine slot
-  uint32_t token[256];                  // kNoSignal: none
-  uint32_t group[256];                  // first rank of the token's DP group
+  unsigned long long row_off[kTokens];  // arena offset of each token's combine slot
+  uint32_t token[kTokens];              // kNoSignal: none
+  uint32_t group[kTokens];              // first rank of the token's DP group
   uint32_t q_token[kQueue];
   uint32_t q_group_units[kQueue];
 };
@@ -98,8 +99,9 @@ __device__ __forceinline__ bool wait_tile_sources(const A2AParams& p, int expert
 }
 
 // One fence, then the queued adds on the tokens' arrival counters (one warp).
-__device__ __forceinline__ void flush(const A2AParams& p, const PeerStage* st, uint32_t count,
-                                      int lane) {
+template <int kTokens>
+__device__ __forceinline__ void flush(const A2AParams& p, const PeerStage<kTokens>* st,
+                                      uint32_t count, int lane) {
   ptx::fence_acq_rel_sys();
   for (uint32_t i = lane; i < count; i += 32) {
     const uint32_t grp = st->q_group_units[i] & 0xffu;

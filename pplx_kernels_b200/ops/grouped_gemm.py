@@ -22,9 +22,10 @@ def grouped_gemm(x: torch.Tensor, w: torch.Tensor, counts: torch.Tensor,
                  half_n: int = 0, cta_pair: int = -1) -> torch.Tensor:
     """x: [E, rows, K] bf16, w: [E, N or 2N, K] bf16, counts: [E] int32 -> out [E, rows, N] bf16.
 
-    ``half_n`` (0 = 128) limits a tile to ``2 * half_n`` token rows, the columns of its
-    accumulator; up to that limit the kernel picks the number of tiles from the row counts it
-    reads on the device, so ``expected_rows`` is only kept for callers that pass it.
+    ``expected_rows`` (total valid rows, 0 = capacity) is a hint: from 224 rows per expert on, the
+    form with tiles of up to 512 instead of 256 token rows is taken.  The number of tiles follows
+    from the row counts that the kernel reads on the device; ``half_n`` (0 = choose) limits a tile
+    to ``2 * half_n`` token rows, the columns of its accumulator.
     ``cta_pair`` selects the kernel form: 0 = one CTA per tile of 128 weight rows, otherwise two
     CTAs share a tile of 256 weight rows (tcgen05 ``cta_group::2``, less traffic into shared
     memory per flop).

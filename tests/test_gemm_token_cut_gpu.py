@@ -21,6 +21,7 @@ RTOL, ATOL = 2.0 ** -8, 2e-4
     ([1, 15, 16, 17, 31, 32, 33, 0], 136, 72, 0),
     ([255, 256, 257, 1], 64, 264, 0),
     ([1030, 7, 513], 72, 136, 0),       # five unequal tiles beside a single narrow one
+    ([512, 481, 289, 256], 200, 264, 0),  # two MMAs per tile, equal and unequal
     ([300, 65, 0, 1], 320, 8, 16),      # the narrowest limit: ten tiles of 32 rows
 ])
 def test_token_cut(swiglu, cta_pair, counts, K, N, half_n):
