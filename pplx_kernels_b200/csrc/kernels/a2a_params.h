@@ -102,8 +102,8 @@ struct A2AParams {
   uint32_t* recv_count;   // [nle] rows received per local expert by the last dispatch
   uint2* row_src;         // [nle][cap] {src_rank | k << 16, src_token} per received row
   uint2* row_of;          // world of one rank: [max_tokens * topk] {local expert, row} of every
-                          //     (token, k) of the last dispatch, {kNoRow, 0} where it has none;
-                          //     nullptr otherwise
+                          //     (token, k) of the last dispatch (packed or not), {kNoRow, 0}
+                          //     where it has none; nullptr otherwise
   Status* status;
   uint64_t timeout_ns;
   uint64_t* trace;        // optional [kTraceSlots] %globaltimer stamps of block 0, or null

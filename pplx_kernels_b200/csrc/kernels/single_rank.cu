@@ -15,6 +15,11 @@
 //  * dispatch leaves (local expert, row) of every (token, k) in `row_of`, and combine gathers
 //    the top-k rows of each token from expert_y itself and writes the weighted sum.
 //
+// Every form of dispatch leaves both directions of that table behind: `row_of` for combine, and
+// (token, k) of every row in `row_src` for the peer-storing down projection (after the packed send
+// the staging-fed up projection writes that one), so that either half of the fused path goes
+// with the other half of the plain one.
+//
 // Both are bound by DRAM from a few hundred tokens on and by launch plus two dependent memory
 // round trips below that.  DeepSeek-V3 shape, fp8 in, bf16 out, kernel times before and after:
 // 4096 tokens 215 -> 58 us (272 MB) and 274 -> 110 us (529 MB); 128 tokens 14.2 -> 6.8 and
@@ -269,7 +274,18 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
         sm.place[j] = place;
         sm.off[j] = off;
       }
-      if (kForm != kPacked && owner) p.row_of[static_cast<size_t>(tb) * topk + j] = place;
+      if (owner) {
+        uint2 kept = place;
+        if constexpr (kForm == kPacked) {
+          // (The slot exists, but expert_y has no row for it.)
+          if (place.y >= static_cast<uint32_t>(p.cap)) kept = make_uint2(kNoRow, 0u);
+        } else if (place.x != kNoRow) {
+          p.row_src[static_cast<size_t>(e) * p.cap + place.y] =
+              make_uint2(static_cast<uint32_t>(p.rank) | static_cast<uint32_t>(j % topk) << 16,
+                         static_cast<uint32_t>(i));
+        }
+        p.row_of[static_cast<size_t>(tb) * topk + j] = kept;
+      }
     }
     __syncthreads();
     if (tb == t0) stamp(p, kTrDispatchPosted, kTrDispatchPosted);
