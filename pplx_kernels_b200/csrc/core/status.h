@@ -24,7 +24,8 @@ enum StatusCode : uint32_t {
   kBadExpert = 2,     // an expert index >= num_experts
   kSlotOverflow = 3,  // a sender reserved a staging slot beyond its region
   kRowOverflow = 4,   // a receiver reserved an output row beyond the capacity
-  kBadToken = 5,      // a trailer named a token index >= max_num_tokens
+  kBadToken = 5,      // a trailer named a token index >= max_num_tokens, or combine was given a token
+                      // that the dispatch before it did not have
   kOutOfOrder = 6,    // two dispatches (or two combines) in a row on one object
 };
 

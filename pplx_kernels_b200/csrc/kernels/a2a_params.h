@@ -104,6 +104,7 @@ struct A2AParams {
   uint2* row_of;          // world of one rank: [max_tokens * topk] {local expert, row} of every
                           //     (token, k) of the last dispatch (packed or not), {kNoRow, 0}
                           //     where it has none; nullptr otherwise
+  uint32_t* dispatched;   // world of one rank: tokens of the last dispatch
   Status* status;
   uint64_t timeout_ns;
   uint64_t* trace;        // optional [kTraceSlots] %globaltimer stamps of block 0, or null

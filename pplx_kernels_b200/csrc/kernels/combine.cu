@@ -94,7 +94,7 @@ __device__ __forceinline__ void trace_block(const A2AParams& p, int first_slot) 
 // ---- phases --------------------------------------------------------------------
 
 template <typename T, bool kLines>
-__device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSmem& sm, int m) {
+__device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSmem& sm) {
   const A2AParams& p = a.p;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -112,7 +112,7 @@ __device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSm
   }
   trace(p, kTrCombineLayout);
   const uint32_t total_rows =
-      by_token ? static_cast<uint32_t>(m) * static_cast<uint32_t>(p.topk) : sm.estart[p.nle];
+      by_token ? *p.dispatched * static_cast<uint32_t>(p.topk) : sm.estart[p.nle];
   // {local expert, row} of the f-th row and {source rank | k << 16, token} of its origin.
   auto find_row = [&](uint32_t f, uint2& place, uint2& rs) {
     if (by_token) {
@@ -419,8 +419,10 @@ __device__ __forceinline__ void recv_phase(const CombineArgs& a, const CombineSm
   const uint32_t complete = ptx::ld_volatile(p.comb_iter) * per_round;
   if (blockIdx.x == 0) {
     // Tokens beyond bound_m receive nothing in this combine; advance their counters
-    // here so that every counter grows by the same amount per combine.
-    for (int i = m + tid; i < p.max_tokens; i += blockDim.x) atomicAdd(arrived + i, per_round);
+    // here so that every counter grows by the same amount per combine.  (In a world of one rank
+    // the send half has sent whatever was dispatched, also beyond a smaller bound_m of this call.)
+    const int first = p.row_of != nullptr ? max(m, static_cast<int>(*p.dispatched)) : m;
+    for (int i = first + tid; i < p.max_tokens; i += blockDim.x) atomicAdd(arrived + i, per_round);
   }
   const uint32_t gwarp = blockIdx.x * nwarps + warp;
   const uint32_t gwarps = gridDim.x * nwarps;
@@ -480,7 +482,7 @@ __device__ __forceinline__ void combine_body(const CombineArgs& a, uint32_t* sme
   m = min(m, p.max_tokens);
   trace(p, kTrCombineStart);
   trace_block(p, kTrBlockCombineStart);
-  if constexpr (SEND) send_phase<T, kLines>(a, sm, m);
+  if constexpr (SEND) send_phase<T, kLines>(a, sm);
   trace(p, kTrCombineSent);
   if constexpr (SEND && RECV) __syncthreads();
   if constexpr (RECV) {

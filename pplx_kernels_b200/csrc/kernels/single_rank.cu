@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
     if (started != iter_now)
       report_failure(p.status, kOutOfOrder, kPhaseDispatchCounts, 0, iter_now, started, p.rank);
     *p.comb_iter = started + 1u;
+    *p.dispatched = static_cast<uint32_t>(m);
     if constexpr (kForm == kStage) {
       // Tokens staged by this half, + 1.  (Rows per expert travel in recv_count.)
       ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(p.peer[p.rank] + p.off_counts) +
@@ -485,6 +486,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
   const uint32_t chunks = static_cast<uint32_t>((nvec8 + 32 * kVec - 1) / (32 * kVec));
   const uint32_t total = static_cast<uint32_t>(m) * chunks;
   const uint32_t gwarps = gridDim.x * kWarps;
+  const uint32_t dispatched = ptx::ld_volatile(p.dispatched);
   stamp(p, kTrCombineStart, kTrCombineSent);
   stamp_block(p, kTrBlockCombineStart);
 
@@ -553,6 +555,12 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
           for (int q = 0; q < kVec; ++q) x[q][j].fma_into(acc[q], w[j]);
         }
       }
+    }
+    if (static_cast<uint32_t>(i) >= dispatched) {
+      // What row_of says of this token is left from an earlier dispatch.
+      if (lane == 0)
+        report_failure(p.status, kBadToken, kPhaseCombinePayload, i, dispatched, m, p.rank);
+      continue;
     }
     if (!whole) {
       // An entry of this token named no expert: the token has no result.

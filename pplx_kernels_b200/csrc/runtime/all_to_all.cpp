@@ -159,7 +159,7 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
     params_.mc_combine = possible && (forced > 0 || (forced < 0 && params_.world >= 4)) ? 1 : 0;
   }
 
-  iter_ = DeviceBuffer<uint32_t>(2);
+  iter_ = DeviceBuffer<uint32_t>(3);
   recv_count_ = DeviceBuffer<uint32_t>(params_.nle);
   // (A world of one rank also keeps where each (token, k) went, behind row_src.)
   const size_t rows = static_cast<size_t>(params_.nle) * params_.cap;
@@ -177,6 +177,7 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
   params_.trace = nullptr;
   params_.iter = iter_.get();
   params_.comb_iter = iter_.get() + 1;
+  params_.dispatched = iter_.get() + 2;
   params_.recv_count = recv_count_.get();
   params_.row_src = row_src_.get();
   params_.row_of = single ? row_src_.get() + rows : nullptr;

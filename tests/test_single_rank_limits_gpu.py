@@ -1,0 +1,82 @@
+"""World of one rank: what the calls report and keep to where the input goes past a limit."""
+
+import pytest
+import torch
+
+import pplx_kernels_b200 as pk
+from pplx_kernels_b200.utils.testing import MoEConfig
+from pplx_kernels_b200.utils.verify import RankBuffers, world_inputs
+
+pytestmark = pytest.mark.gpu
+
+HALVES = ({"do_recv": False}, {"do_send": False})
+
+
+def _object(cfg: MoEConfig, seed: int, num_tokens: int):
+    ata = pk.AllToAll.intranode(cfg.max_num_tokens, cfg.num_experts, cfg.experts_per_token, 0, 1, 1,
+                                cfg.hidden_dim, cfg.hidden_dim_bytes, cfg.hidden_dim_scale_bytes)
+    ata.set_timeout_ms(300)
+    inputs = world_inputs(cfg, 1, 1, seed=seed, num_tokens=num_tokens)
+    return ata, inputs, RankBuffers(cfg, 1, 1, inputs[0], torch.device("cuda", 0))
+
+
+def _dispatch(ata, buf, split):
+    for kw in HALVES if split else ({},):
+        ata.dispatch(buf.counts, buf.expert_x, buf.expert_scale, buf.x, buf.x_scale, buf.indices,
+                     buf.bound_m, **kw)
+
+
+def _combine(ata, buf, split, bound_m=None):
+    for kw in HALVES if split else ({},):
+        ata.combine(buf.out, buf.indices, buf.weights, buf.expert_y,
+                    buf.bound_m if bound_m is None else bound_m, **kw)
+
+
+@pytest.mark.parametrize("lines", [0, 1])
+@pytest.mark.parametrize("split", [False, True])
+def test_combine_of_more_tokens_than_dispatched_is_reported(split, lines, monkeypatch):
+    """The places of the extra tokens are those of an earlier pass: their sums are not results."""
+    monkeypatch.setenv("PPLX_B200_LL", str(lines))
+    cfg = MoEConfig(num_experts=8, experts_per_token=2, hidden_dim=64, max_num_tokens=12)
+    ata, _, buf = _object(cfg, 3, 12)
+    _dispatch(ata, buf, split)
+    buf.make_expert_y()
+    _combine(ata, buf, split)
+    buf.bound_m.view(torch.int32).fill_(5)
+    _dispatch(ata, buf, split)
+    torch.cuda.synchronize()
+    ata.check_status()
+    buf.out.fill_(float("nan"))
+    more = torch.full((1,), 12, dtype=torch.int32, device=buf.out.device).view(torch.uint32)
+    _combine(ata, buf, split, bound_m=more)
+    torch.cuda.synchronize()
+    assert ata.status()["code"] != 0
+    out = buf.out.float()
+    assert torch.isnan(out[5:]).all()
+    if not split:
+        assert not torch.isnan(out[:5]).any()
+    ata.destroy()
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("lines", [0, 1])
+def test_combine_of_fewer_tokens_than_dispatched(split, lines, monkeypatch):
+    """The rest of the tokens is left alone, and the next pass of all of them is whole."""
+    monkeypatch.setenv("PPLX_B200_LL", str(lines))
+    cfg = MoEConfig(num_experts=8, experts_per_token=2, hidden_dim=64, max_num_tokens=12)
+    ata, inputs, buf = _object(cfg, 4, 12)
+    fewer = torch.full((1,), 5, dtype=torch.int32, device=buf.out.device).view(torch.uint32)
+    whole = None
+    for bound_m in (None, fewer, None, fewer, None):
+        _dispatch(ata, buf, split)
+        buf.make_expert_y()
+        buf.out.fill_(float("nan"))
+        _combine(ata, buf, split, bound_m)
+        torch.cuda.synchronize()
+        ata.check_status()
+        m = 12 if bound_m is None else 5
+        if whole is None:
+            whole = buf.out.clone()
+        assert torch.equal(buf.out[:m], whole[:m])
+        assert torch.isnan(buf.out[m:].float()).all()
+    ata.destroy()
