@@ -16,6 +16,13 @@ __device__ __forceinline__ void reset_packed_flags(const A2AParams& p, int parit
   for (int i = threadIdx.x; i < p.nle * p.world; i += blockDim.x) arrived_e[i] = 0;
 }
 
+// World of one rank, in a combine: tokens of the dispatch it belongs to.  (Dispatch number n,
+// counted from 1 in comb_iter, had the parity of n - 1.)
+__device__ __forceinline__ uint32_t last_dispatched(const A2AParams& p) {
+  const uint4 state = __ldcg(reinterpret_cast<const uint4*>(p.iter));
+  return (state.y & 1u) != 0u ? state.z : state.w;
+}
+
 // First step of a combine (all threads of one block call it): the dispatch that produced the
 // rows has finished on this rank, so clear the flag set it used and move on to the other one.
 // No peer can write this set again before it has seen counts of this rank's next dispatch.

@@ -96,15 +96,16 @@ struct A2AParams {
   uint8_t* mc;  // NVLink multicast alias of the arenas (same offsets on all ranks), or nullptr
   int mc_combine;  // non-zero: the counter-form combine multicasts rows (tokens replicated on all ranks)
 
-  // rank-local state (plain device memory)
+  // rank-local state (plain device memory); iter, comb_iter and dispatched are one 16-byte vector
   uint32_t* iter;         // dispatch iteration counter; its parity selects the flag set
   uint32_t* comb_iter;    // number of dispatches started = ordinal of the coming combine
   uint32_t* recv_count;   // [nle] rows received per local expert by the last dispatch
   uint2* row_src;         // [nle][cap] {src_rank | k << 16, src_token} per received row
   uint2* row_of;          // world of one rank: [max_tokens * topk] {local expert, row} of every
-                          //     (token, k) of the last dispatch (packed or not), {kNoRow, 0}
-                          //     where it has none; nullptr otherwise
-  uint32_t* dispatched;   // world of one rank: tokens of the last dispatch
+                          //     (token, k) of the last dispatch (packed or not), {kNoRow, *}
+                          //     where it has none and for all tokens it did not have; nullptr
+                          //     otherwise
+  uint32_t* dispatched;   // world of one rank: [2] tokens of the last dispatch of each parity
   Status* status;
   uint64_t timeout_ns;
   uint64_t* trace;        // optional [kTraceSlots] %globaltimer stamps of block 0, or null

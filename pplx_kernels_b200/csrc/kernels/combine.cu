@@ -112,7 +112,7 @@ __device__ __forceinline__ void send_phase(const CombineArgs& a, const CombineSm
   }
   trace(p, kTrCombineLayout);
   const uint32_t total_rows =
-      by_token ? *p.dispatched * static_cast<uint32_t>(p.topk) : sm.estart[p.nle];
+      by_token ? last_dispatched(p) * static_cast<uint32_t>(p.topk) : sm.estart[p.nle];
   // {local expert, row} of the f-th row and {source rank | k << 16, token} of its origin.
   auto find_row = [&](uint32_t f, uint2& place, uint2& rs) {
     if (by_token) {
@@ -421,7 +421,7 @@ __device__ __forceinline__ void recv_phase(const CombineArgs& a, const CombineSm
     // Tokens beyond bound_m receive nothing in this combine; advance their counters
     // here so that every counter grows by the same amount per combine.  (In a world of one rank
     // the send half has sent whatever was dispatched, also beyond a smaller bound_m of this call.)
-    const int first = p.row_of != nullptr ? max(m, static_cast<int>(*p.dispatched)) : m;
+    const int first = p.row_of != nullptr ? max(m, static_cast<int>(last_dispatched(p))) : m;
     for (int i = first + tid; i < p.max_tokens; i += blockDim.x) atomicAdd(arrived + i, per_round);
   }
   const uint32_t gwarp = blockIdx.x * nwarps + warp;

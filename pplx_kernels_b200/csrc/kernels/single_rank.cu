@@ -183,14 +183,18 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
   uint32_t u = u0 + warp;
   load(u);
 
-  const int parity = static_cast<int>(ptx::ld_volatile(p.iter) & 1u);
+  // {iter, comb_iter, dispatched[0], dispatched[1]}; of these, this kernel changes the second and
+  // the third or fourth, which are not used from here.
+  const uint4 state = __ldcg(reinterpret_cast<const uint4*>(p.iter));
+  const int parity = static_cast<int>(state.x & 1u);
+  const uint32_t dispatched_before = parity != 0 ? state.z : state.w;
   if (blk == 0 && tid == 0) {
     // A new round begins; dispatches started must equal combines finished.
     const uint32_t iter_now = *p.iter, started = *p.comb_iter;
     if (started != iter_now)
       report_failure(p.status, kOutOfOrder, kPhaseDispatchCounts, 0, iter_now, started, p.rank);
     *p.comb_iter = started + 1u;
-    *p.dispatched = static_cast<uint32_t>(m);
+    p.dispatched[parity] = static_cast<uint32_t>(m);
     if constexpr (kForm == kStage) {
       // Tokens staged by this half, + 1.  (Rows per expert travel in recv_count.)
       ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(p.peer[p.rank] + p.off_counts) +
@@ -371,6 +375,11 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
       __syncthreads();
     }
   }
+  if (last_block) {
+    // Tokens that the dispatch before had and this one does not.
+    for (uint32_t j = static_cast<uint32_t>(m) * topk + tid; j < dispatched_before * topk; j += kThreads)
+      p.row_of[j] = make_uint2(kNoRow, 0u);
+  }
   stamp(p, kTrDispatchStored, kTrDispatchStored);
 
   if constexpr (kForm == kPacked) {
@@ -486,7 +495,6 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
   const uint32_t chunks = static_cast<uint32_t>((nvec8 + 32 * kVec - 1) / (32 * kVec));
   const uint32_t total = static_cast<uint32_t>(m) * chunks;
   const uint32_t gwarps = gridDim.x * kWarps;
-  const uint32_t dispatched = ptx::ld_volatile(p.dispatched);
   stamp(p, kTrCombineStart, kTrCombineSent);
   stamp_block(p, kTrBlockCombineStart);
 
@@ -556,16 +564,14 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
         }
       }
     }
-    if (static_cast<uint32_t>(i) >= dispatched) {
-      // What row_of says of this token is left from an earlier dispatch.
-      if (lane == 0)
-        report_failure(p.status, kBadToken, kPhaseCombinePayload, i, dispatched, m, p.rank);
-      continue;
-    }
     if (!whole) {
-      // An entry of this token named no expert: the token has no result.
-      if (lane == 0)
-        report_failure(p.status, kBadExpert, kPhaseCombinePayload, i, topk, 0, p.rank);
+      // The token was not dispatched, or an entry of it named no expert: it has no result.
+      if (lane == 0) {
+        const uint32_t had = last_dispatched(p);
+        const bool known = static_cast<uint32_t>(i) < had;
+        report_failure(p.status, known ? kBadExpert : kBadToken, kPhaseCombinePayload, i,
+                       known ? topk : had, known ? 0 : i, p.rank);
+      }
       continue;
     }
 #pragma unroll

@@ -159,7 +159,7 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
     params_.mc_combine = possible && (forced > 0 || (forced < 0 && params_.world >= 4)) ? 1 : 0;
   }
 
-  iter_ = DeviceBuffer<uint32_t>(3);
+  iter_ = DeviceBuffer<uint32_t>(4);
   recv_count_ = DeviceBuffer<uint32_t>(params_.nle);
   // (A world of one rank also keeps where each (token, k) went, behind row_src.)
   const size_t rows = static_cast<size_t>(params_.nle) * params_.cap;
@@ -181,6 +181,7 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
   params_.recv_count = recv_count_.get();
   params_.row_src = row_src_.get();
   params_.row_of = single ? row_src_.get() + rows : nullptr;
+  forget_rows();
   params_.status = status_.get();
   params_.timeout_ns = static_cast<uint64_t>(env_long("PPLX_B200_TIMEOUT_MS", 10000)) * 1000000ull;
   params_.debug_checks = env_long("PPLX_B200_DEBUG_CHECKS", 0) != 0 ? 1 : 0;
@@ -303,6 +304,11 @@ void AllToAll::begin(Step first, bool both) {
   if (both) advance(static_cast<Step>(static_cast<int>(first) + 1));
 }
 
+void AllToAll::forget_rows() {
+  if (params_.row_of == nullptr) return;
+  CUDA_CHECK(cudaMemset(params_.row_of, 0xff, sizeof(uint2) * params_.max_tokens * params_.topk));
+}
+
 void AllToAll::reset() {
   CUDA_CHECK(cudaDeviceSynchronize());
   uint8_t* mine = params_.peer[cfg_.rank];
@@ -314,6 +320,7 @@ void AllToAll::reset() {
   }
   CUDA_CHECK(cudaMemset(iter_.get(), 0, iter_.bytes()));
   CUDA_CHECK(cudaMemset(recv_count_.get(), 0, recv_count_.bytes()));
+  forget_rows();
   Status init{};
   init.mirror = reinterpret_cast<unsigned long long>(status_host_.device_ptr());
   status_.copy_from_host(&init, 1);

@@ -205,6 +205,7 @@ class AllToAll {
 
   DispatchArgs make_dispatch_args(const DispatchCall& call) const;
   CombineArgs make_combine_args(const CombineCall& call) const;
+  void forget_rows();       // world of one rank: no token has a row
   int block_limit() const;  // blocks a launch may have at most
   int dispatch_grid(int num_tokens) const;
   int combine_grid(int num_tokens) const;
