@@ -888,6 +888,20 @@ std::vector<int64_t> wait_probe_op(const at::Tensor& flag, double timeout_ms) {
   });
 }
 
+std::vector<int64_t> mbar_wait_probe_op(const at::Tensor& device_of, double limit_ms) {
+  TORCH_CHECK(device_of.is_cuda(), "a CUDA tensor says which device to probe");
+  TORCH_CHECK(limit_ms > 0 && limit_ms <= 2000, "the limit must be in (0, 2000] milliseconds");
+  const c10::cuda::OptionalCUDAGuard guard(device_of.device());
+  return guarded([&] {
+    DeviceBuffer<uint64_t> result(2);
+    auto stream = at::cuda::getCurrentCUDAStream();
+    CUDA_CHECK(launch_mbar_wait_probe(result.get(), static_cast<uint32_t>(limit_ms * 1e6), stream));
+    CUDA_CHECK(cudaStreamSynchronize(stream));
+    const std::vector<uint64_t> r = result.to_host();
+    return std::vector<int64_t>(r.begin(), r.end());
+  });
+}
+
 }  // namespace
 
 void register_all_to_all_ops(torch::Library& m) {
@@ -999,6 +1013,7 @@ void register_symmetric_memory_ops(torch::Library& m) {
         &fd_exchange_selftest_op);
   m.def("sleep_on_stream(float seconds) -> ()", &sleep_on_stream_op);
   m.def("wait_probe(Tensor flag, float timeout_ms) -> int[]", &wait_probe_op);
+  m.def("mbar_wait_probe(Tensor device_of, float limit_ms) -> int[]", &mbar_wait_probe_op);
 }
 
 }  // namespace pplx

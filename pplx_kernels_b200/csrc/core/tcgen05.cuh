@@ -63,21 +63,25 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
-// Waits for the phase with the given parity to complete, for at most about `limit_ns`.
+// Waits for the phase with the given parity to complete, for at most `limit_ns` (below 2^31) and
+// two sleeps.
 // `abort_flag` is a shared-memory word that any role of the CTA sets when it
 // gives up; once set, every wait returns false at its next check so that the CTA
 // drains to its teardown instead of hanging.
 //
 // The thread sleeps in the barrier unit (a try_wait with a time hint of a millisecond) and is
-// woken by the phase itself; the limit counts those sleeps.  Polling instead, with a look at
-// %globaltimer in between, woke up about a microsecond late and kept the issue slots and the
-// shared-memory port busy that the working warps of the CTA need.
+// woken by the phase itself.  Polling instead, with a look at %globaltimer every few polls, woke
+// up about a microsecond late and kept the issue slots and the shared-memory port busy that the
+// working warps of the CTA need.  How long a sleep in vain lasts is up to the hardware (0.07 to
+// 0.7 ms were measured), so the limit is read off the clock, after such a sleep.  (Modulo 2^32 ns,
+// with an odd end so that 0 can say that there is none yet: a wide clock cost registers.)
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          volatile uint32_t* abort_flag, uint64_t limit_ns) {
+                                           volatile uint32_t* abort_flag, uint32_t limit_ns) {
   if (mbar_try_wait(bar, parity)) return true;
   constexpr uint32_t kSleepNs = 1000000;
+  uint32_t end = 0;
 #pragma unroll 1
-  for (uint64_t slept = 0; slept < limit_ns; slept += kSleepNs) {
+  while (true) {
     uint32_t done;
     asm volatile(
         "{\n\t"
@@ -90,9 +94,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
         : "memory");
     if (done != 0u) return true;
     if (*abort_flag != 0u) return false;
+    uint32_t now;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(now));
+    if (end == 0u) {
+      end = (now + limit_ns) | 1u;
+    } else if (static_cast<int32_t>(now - end) > 0) {
+      *abort_flag = 1u;
+      return false;
+    }
   }
-  *abort_flag = 1u;
-  return false;
 }
 
 // ----------------------------------------------------------------- TMA ----

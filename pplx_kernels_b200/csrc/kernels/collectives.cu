@@ -1,6 +1,7 @@
 #include "collectives.h"
 
 #include "../core/ptx.cuh"
+#include "../core/tcgen05.cuh"
 #include "../core/wait.cuh"
 
 namespace pplx {
@@ -72,6 +73,32 @@ __global__ void wait_probe_kernel(const uint32_t* flag, Status* status, uint64_t
   wait_until(flag, PredNonZero{}, seen, w, kPhaseTest, 0u, 1u);
 }
 
+// Warp 0 waits, warp 1 arrives 32 * kProbeArrivals times: one too few for the phase.
+constexpr int kProbeArrivals = 256;
+
+__global__ void mbar_wait_probe_kernel(uint64_t* result, uint32_t limit_ns) {
+  __shared__ uint64_t bar;
+  __shared__ uint32_t abort_flag;
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    tc::mbar_init(&bar, 32 * kProbeArrivals + 1);
+    tc::fence_mbar_init();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const uint64_t t0 = ptx::globaltimer_ns();
+    const bool ok = tc::mbar_wait(&bar, 0, &abort_flag, limit_ns);
+    result[1] = ptx::globaltimer_ns() - t0;
+    result[0] = ok ? 1 : 0;
+  } else if (threadIdx.x >= 32) {
+    for (int i = 0; i < kProbeArrivals; ++i) {
+      tc::mbar_arrive(&bar);
+      ptx::nanosleep(1000);
+    }
+  }
+  __syncthreads();
+}
+
 }  // namespace
 
 cudaError_t launch_barrier(const BarrierParams& b, cudaStream_t stream) {
@@ -94,6 +121,11 @@ cudaError_t launch_sleep(uint64_t ns, cudaStream_t stream) {
 cudaError_t launch_wait_probe(const uint32_t* flag, Status* status, uint64_t timeout_ns,
                               cudaStream_t stream) {
   wait_probe_kernel<<<1, 1, 0, stream>>>(flag, status, timeout_ns);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mbar_wait_probe(uint64_t* result, uint32_t limit_ns, cudaStream_t stream) {
+  mbar_wait_probe_kernel<<<1, 64, 0, stream>>>(result, limit_ns);
   return cudaGetLastError();
 }
 

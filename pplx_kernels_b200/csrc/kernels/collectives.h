@@ -52,4 +52,9 @@ cudaError_t launch_sleep(uint64_t ns, cudaStream_t stream);
 cudaError_t launch_wait_probe(const uint32_t* flag, Status* status, uint64_t timeout_ns,
                               cudaStream_t stream);
 
+// One thread waits (bounded by `limit_ns`) for a shared-memory barrier whose phase never
+// completes, while others arrive on it.  result[0]: 1 if the wait succeeded all the same,
+// result[1]: nanoseconds it took.
+cudaError_t launch_mbar_wait_probe(uint64_t* result, uint32_t limit_ns, cudaStream_t stream);
+
 }  // namespace pplx

@@ -50,7 +50,7 @@ constexpr int kUmmaKBytes = 32;
 constexpr int kThreads = 384;
 constexpr int kTmemCols = 512;
 constexpr int kPeerTokens = 256;   // at least the widest token tile
-constexpr uint64_t kWaitLimitNs = 2000000000ull;
+constexpr uint32_t kWaitLimitNs = 2000000000u;
 constexpr int kMaxExperts = 1024;
 
 __device__ __forceinline__ float silu(float v) { return v / (1.0f + __expf(-v)); }

@@ -87,7 +87,7 @@ constexpr int kThreads = 384;
 constexpr int kTmemCols = 512;    // an accumulator of kMaxTokens columns, or two of half of them
 constexpr uint32_t kRowBytes = kBlockK * 2;
 constexpr uint32_t kWBytes = kBlockM * kRowBytes;
-constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s per wait
+constexpr uint32_t kWaitLimitNs = 2000000000u;  // 2 s per wait
 constexpr int kMaxExperts = 1024;
 constexpr int kDrainPlain = 8;    // cycles per token row to read out an accumulator that is the only
 constexpr int kDrainSwiglu = 35;  // one, as fitted to the times of both widths at 512 rows
