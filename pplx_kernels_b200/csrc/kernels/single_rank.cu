@@ -50,7 +50,7 @@ namespace {
 
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kBlocksPerSm = 2;       // 64 registers per thread
+constexpr int kBlocksPerSm = kSingleRankBlocksPerSm;  // 64 registers per thread
 constexpr int kMinEntries = 512;  // (token, k) entries whose rows a block knows at a time
 
 enum Form : int {
@@ -612,10 +612,11 @@ cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, 
                                    cudaStream_t stream) {
   const bool quant = a.quantize != 0;
   const int64_t units = static_cast<int64_t>(a.num_tokens) * chunks_of(a.p, quant);
+  const int one_per_sm = std::min(limit, get_sm_count());
   if (!send) {
     int chunks_sent = chunks_of(a.p, quant);
     void* params[] = {const_cast<DispatchArgs*>(&a), &chunks_sent};
-    return launch(reinterpret_cast<const void*>(&single_unstage_kernel), grid_for(units, limit), 0,
+    return launch(reinterpret_cast<const void*>(&single_unstage_kernel), grid_for(units, one_per_sm), 0,
                   params, stream);
   }
   const void* fn;
@@ -631,8 +632,8 @@ cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, 
   }
   void* params[] = {const_cast<DispatchArgs*>(&a)};
   // (Staging stores a chunk once, not top-k times: twice the blocks only count twice.)
-  const int grid = a.packed ? std::clamp(a.num_tokens, 1, limit)
-                            : grid_for(units, recv ? kBlocksPerSm * limit : limit);
+  const int grid = a.packed ? std::clamp(a.num_tokens, 1, one_per_sm)
+                            : grid_for(units, recv ? limit : one_per_sm);
   return launch(fn, grid, dispatch_smem(a.p), params, stream);
 }
 
@@ -641,9 +642,9 @@ cudaError_t launch_single_combine(const CombineArgs& a, DType in, DType out, int
   const int vecs = ((a.p.hidden_dim >> 3) + 31) / 32;
   // Two vectors per lane where a token has few rows and there are enough tokens to keep every
   // warp at work all the same: with top-2 one vector is two 16-byte loads in flight per lane.
-  const bool pairs = a.p.topk <= 4 && static_cast<int64_t>(a.num_tokens) * vecs >= 4 * kWarps * limit;
+  const bool pairs = a.p.topk <= 4 && static_cast<int64_t>(a.num_tokens) * vecs >= 2 * kWarps * limit;
   const int64_t units = static_cast<int64_t>(a.num_tokens) * (pairs ? (vecs + 1) / 2 : vecs);
-  const int grid = grid_for(units, kBlocksPerSm * limit);
+  const int grid = grid_for(units, limit);
   return dispatch_types(in, out, [&]<typename T, typename U>() {
     void* params[] = {const_cast<CombineArgs*>(&a)};
     const void* fn = pairs ? reinterpret_cast<const void*>(&single_combine_kernel<T, U, 2>)

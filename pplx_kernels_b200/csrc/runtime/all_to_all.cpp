@@ -344,8 +344,8 @@ void AllToAll::set_timeout_ms(double ms) {
   params_.timeout_ns = static_cast<uint64_t>(ms * 1e6);
 }
 
-int AllToAll::block_limit() const {
-  return max_blocks_ > 0 ? std::min(max_blocks_, num_sms_) : num_sms_;
+int AllToAll::block_limit(int per_sm) const {
+  return max_blocks_ > 0 ? std::min(max_blocks_, per_sm * num_sms_) : per_sm * num_sms_;
 }
 
 int AllToAll::dispatch_grid(int num_tokens) const {
@@ -460,7 +460,7 @@ void AllToAll::dispatch_send_packed(const DispatchCall& call, cudaStream_t strea
   const DispatchArgs a = make_packed_send_args(call);
   begin(Step::kDispatchSend, false);
   if (cfg_.world_size == 1) {
-    CUDA_CHECK(launch_single_dispatch(a, true, false, block_limit(), stream));
+    CUDA_CHECK(launch_single_dispatch(a, true, false, block_limit(kSingleRankBlocksPerSm), stream));
     return;
   }
   CUDA_CHECK(launch_dispatch(a, true, false, dispatch_grid(call.num_tokens), stream));
@@ -525,7 +525,7 @@ void AllToAll::dispatch(const DispatchCall& call, SplitMode mode, cudaStream_t s
   const bool send = mode != SplitMode::kRecv, recv = mode != SplitMode::kSend;
   begin(send ? Step::kDispatchSend : Step::kDispatchRecv, send && recv);
   if (cfg_.world_size == 1) {
-    CUDA_CHECK(launch_single_dispatch(a, send, recv, block_limit(), stream));
+    CUDA_CHECK(launch_single_dispatch(a, send, recv, block_limit(kSingleRankBlocksPerSm), stream));
     return;
   }
   if (params_.tiny != 0 && !call.quantize) {
@@ -543,7 +543,8 @@ void AllToAll::combine(const CombineCall& call, SplitMode mode, cudaStream_t str
   begin(send ? Step::kCombineSend : Step::kCombineRecv, send && recv);
   if (cfg_.world_size == 1 && send && recv) {
     combine_send_used_lines_ = false;
-    CUDA_CHECK(launch_single_combine(a, call.in, call.out, block_limit(), stream));
+    CUDA_CHECK(launch_single_combine(a, call.in, call.out, block_limit(kSingleRankBlocksPerSm),
+                                     stream));
     return;
   }
   // The receive half follows whatever its send half used: lines for a send of this class,

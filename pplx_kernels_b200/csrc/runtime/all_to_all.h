@@ -206,7 +206,8 @@ class AllToAll {
   DispatchArgs make_dispatch_args(const DispatchCall& call) const;
   CombineArgs make_combine_args(const CombineCall& call) const;
   void forget_rows();       // world of one rank: no token has a row
-  int block_limit() const;  // blocks a launch may have at most
+  // Blocks a launch may have at most: the caller's cap, else `per_sm` for every SM.
+  int block_limit(int per_sm = 1) const;
   int dispatch_grid(int num_tokens) const;
   int combine_grid(int num_tokens) const;
   // Whether a dispatch of this object moves its rows as flag-in-data lines.

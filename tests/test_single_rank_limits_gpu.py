@@ -4,8 +4,9 @@ import pytest
 import torch
 
 import pplx_kernels_b200 as pk
+from pplx_kernels_b200.ops import _ops
 from pplx_kernels_b200.utils.testing import MoEConfig
-from pplx_kernels_b200.utils.verify import RankBuffers, world_inputs
+from pplx_kernels_b200.utils.verify import RankBuffers, verify_dispatch, world_inputs
 
 pytestmark = pytest.mark.gpu
 
@@ -79,4 +80,29 @@ def test_combine_of_fewer_tokens_than_dispatched(split, lines, monkeypatch):
             whole = buf.out.clone()
         assert torch.equal(buf.out[:m], whole[:m])
         assert torch.isnan(buf.out[m:].float()).all()
+    ata.destroy()
+
+
+def _blocks(ata, array: int) -> int:
+    stamps = _ops.all_to_all_read_trace(ata._ptr)
+    return sum(v != 0 for v in stamps[32 + 256 * array: 32 + 256 * (array + 1)])
+
+
+@pytest.mark.parametrize("cap", [0, 1, 7, 150, 400])
+def test_max_blocks_limits_the_blocks_of_a_launch(cap):
+    cfg = MoEConfig(num_experts=64, experts_per_token=8, hidden_dim=4096, max_num_tokens=256)
+    ata, inputs, buf = _object(cfg, 6, 256)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    ata.set_trace(True)
+    ata.set_max_blocks(cap)
+    _dispatch(ata, buf, False)
+    torch.cuda.synchronize()
+    verify_dispatch(cfg, inputs, 1, 0, buf)
+    buf.make_expert_y()
+    _combine(ata, buf, False)
+    torch.cuda.synchronize()
+    ata.check_status()
+    # (The trace holds the stamps of the first 256 blocks.)
+    most = min(256, 2 * sms, cap or 2 * sms)
+    assert 0 < _blocks(ata, 0) <= most and 0 < _blocks(ata, 2) <= most
     ata.destroy()
