@@ -100,6 +100,8 @@ struct A2AParams {
   uint32_t* iter;         // dispatch iteration counter; its parity selects the flag set
   uint32_t* comb_iter;    // number of dispatches started = ordinal of the coming combine
   uint32_t* recv_count;   // [nle] rows received per local expert by the last dispatch
+  uint32_t* recv_total;   // world of one rank: [nle] the same before the limit of `cap` rows, as the
+                          //     send half of a dispatch left it for the receive half
   uint2* row_src;         // [nle][cap] {src_rank | k << 16, src_token} per received row
   uint2* row_of;          // world of one rank: [max_tokens * topk] {local expert, row} of every
                           //     (token, k) of the last dispatch (packed or not), {kNoRow, *}

@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
     // No token follows the last block's: its counts are the totals.
     for (int e = tid; e < E; e += kThreads) {
       if constexpr (kForm == kDirect) a.out_num_tokens[e] = static_cast<int32_t>(sm.base[e]);
+      else p.recv_total[e] = sm.base[e];
       p.recv_count[e] = min(sm.base[e], static_cast<uint32_t>(p.cap));
     }
   }
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
   stamp(p, kTrDispatchCounts, kTrDispatchLayout);
   if (blockIdx.x == 0) {
     for (int e = tid; e < p.nle; e += kThreads)
-      a.out_num_tokens[e] = static_cast<int32_t>(__ldcg(p.recv_count + e));
+      a.out_num_tokens[e] = static_cast<int32_t>(__ldcg(p.recv_total + e));
   }
   const uint32_t total = s_tokens * chunks;
   const uint8_t* stage = p.peer[p.rank] + p.off_disp_stage;

@@ -160,7 +160,7 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
   }
 
   iter_ = DeviceBuffer<uint32_t>(4);
-  recv_count_ = DeviceBuffer<uint32_t>(params_.nle);
+  recv_count_ = DeviceBuffer<uint32_t>(2 * static_cast<size_t>(params_.nle));
   // (A world of one rank also keeps where each (token, k) went, behind row_src.)
   const size_t rows = static_cast<size_t>(params_.nle) * params_.cap;
   const bool single = cfg_.world_size == 1;
@@ -179,6 +179,7 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
   params_.comb_iter = iter_.get() + 1;
   params_.dispatched = iter_.get() + 2;
   params_.recv_count = recv_count_.get();
+  params_.recv_total = recv_count_.get() + params_.nle;
   params_.row_src = row_src_.get();
   params_.row_of = single ? row_src_.get() + rows : nullptr;
   forget_rows();

@@ -106,3 +106,18 @@ def test_max_blocks_limits_the_blocks_of_a_launch(cap):
     most = min(256, 2 * sms, cap or 2 * sms)
     assert 0 < _blocks(ata, 0) <= most and 0 < _blocks(ata, 2) <= most
     ata.destroy()
+
+
+@pytest.mark.parametrize("split", [False, True])
+def test_an_expert_named_twice_by_its_tokens(split):
+    """Counts are those of the routing table in both forms, also beyond the capacity; the rows
+    beyond it are dropped and reported."""
+    cfg = MoEConfig(num_experts=4, experts_per_token=3, hidden_dim=64, max_num_tokens=4)
+    ata, _, buf = _object(cfg, 5, 4)
+    buf.indices = torch.zeros(4, 3, dtype=torch.int32, device=buf.out.device).view(torch.uint32)
+    _dispatch(ata, buf, split)
+    torch.cuda.synchronize()
+    assert buf.counts.tolist() == [12, 0, 0, 0]
+    assert ata.status()["code"] == 4
+    ata.verify_canaries()
+    ata.destroy()
