@@ -117,6 +117,7 @@ struct Smem {
   uint32_t* mine;           // [E] kPacked: rows this block stored per expert
 };
 constexpr unsigned long long kNoOffset = ~0ull;
+constexpr uint32_t kScalesInside = 1u << 31;
 
 __device__ __forceinline__ Smem carve(uint8_t* s, int entries, int E) {
   Smem m;
@@ -196,10 +197,11 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
     *p.comb_iter = started + 1u;
     p.dispatched[parity] = static_cast<uint32_t>(m);
     if constexpr (kForm == kStage) {
-      // Tokens staged by this half, + 1.  (Rows per expert travel in recv_count.)
+      // Tokens staged by this half, + 1, and whether their scales come with their payload: the
+      // receive half may be a call of the other kind.  (Rows per expert travel in recv_count.)
       ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(p.peer[p.rank] + p.off_counts) +
                               a2a_counts_index(p, parity, 0, 0),
-                          static_cast<uint32_t>(m) + 1u);
+                          static_cast<uint32_t>(m) + 1u | (kQuant ? kScalesInside : 0u));
     }
   }
   for (int e = tid; e < E; e += kThreads) {
@@ -405,11 +407,12 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
   }
   if constexpr (kForm == kStage) {
     __syncthreads();
-    // One unit more for the last block: its totals are announced even when there is no token.
-    if (tid == 0 && (u1 > u0 || last_block))
+    // One unit more for the last block, for its totals, and one for the first, for the state of the
+    // object: both are announced even when there is no token.
+    const uint32_t more = (last_block ? 1u : 0u) + (blk == 0 ? 1u : 0u);
+    if (tid == 0 && (u1 - u0) + more > 0)
       ptx::red_add_release_gpu(
-          reinterpret_cast<uint32_t*>(p.peer[p.rank] + p.off_arrived) + parity,
-          (u1 - u0) + (last_block ? 1u : 0u));
+          reinterpret_cast<uint32_t*>(p.peer[p.rank] + p.off_arrived) + parity, (u1 - u0) + more);
   }
   stamp(p, kTrDispatchSignalled, kTrDispatchEnd);
   stamp_block(p, kTrBlockDispatchEnd);
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 
 // Receive half: staged tokens to their rows.
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
-    single_unstage_kernel(const __grid_constant__ DispatchArgs a, int chunks_sent) {
+    single_unstage_kernel(const __grid_constant__ DispatchArgs a) {
   __shared__ uint32_t s_tokens;
   const A2AParams& p = a.p;
   ptx::wait_for_previous_kernels();
@@ -434,7 +437,9 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
     bool ok = wait_until(reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_counts) +
                              a2a_counts_index(p, parity, 0, 0),
                          PredNonZero{}, v, w, kPhaseDispatchCounts, p.rank, 1u);
-    const uint32_t units = ok ? (v - 1u) * chunks_sent + 1u : 0u;
+    const uint32_t sent = (v & kScalesInside) != 0u ? payload_chunks : chunks;
+    v &= ~kScalesInside;
+    const uint32_t units = ok ? (v - 1u) * sent + 2u : 0u;
     ok = ok && wait_until(reinterpret_cast<const uint32_t*>(p.peer[p.rank] + p.off_arrived) + parity,
                           PredGe{units}, seen, w, kPhaseDispatchPayload, p.rank, units);
     s_tokens = ok ? v - 1u : 0u;
@@ -615,8 +620,7 @@ cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, 
   const int64_t units = static_cast<int64_t>(a.num_tokens) * chunks_of(a.p, quant);
   const int one_per_sm = std::min(limit, get_sm_count());
   if (!send) {
-    int chunks_sent = chunks_of(a.p, quant);
-    void* params[] = {const_cast<DispatchArgs*>(&a), &chunks_sent};
+    void* params[] = {const_cast<DispatchArgs*>(&a)};
     return launch(reinterpret_cast<const void*>(&single_unstage_kernel), grid_for(units, one_per_sm), 0,
                   params, stream);
   }

@@ -5,6 +5,7 @@ import torch
 
 import pplx_kernels_b200 as pk
 from pplx_kernels_b200.ops import _ops
+from pplx_kernels_b200.ops.quant import per_token_block_quant
 from pplx_kernels_b200.utils.testing import MoEConfig
 from pplx_kernels_b200.utils.verify import RankBuffers, verify_dispatch, world_inputs
 
@@ -120,4 +121,38 @@ def test_an_expert_named_twice_by_its_tokens(split):
     assert buf.counts.tolist() == [12, 0, 0, 0]
     assert ata.status()["code"] == 4
     ata.verify_canaries()
+    ata.destroy()
+
+
+@pytest.mark.parametrize("quantised_half", ["send", "recv"])
+def test_halves_of_dispatch_and_dispatch_quant(quantised_half):
+    """The receive half takes what the send half staged, whichever call staged it."""
+    dev = torch.device("cuda", 0)
+    cfg = MoEConfig(num_experts=16, experts_per_token=4, hidden_dim=1024, max_num_tokens=600,
+                    in_dtype=torch.float8_e4m3fn)
+    ata, _, buf = _object(cfg, 8, 600)
+    x = torch.randn(600, cfg.hidden_dim, generator=torch.Generator().manual_seed(9)).to(torch.bfloat16)
+    xq, xs = per_token_block_quant(x)
+    quant = (buf.counts, buf.expert_x, buf.expert_scale, x.to(dev), buf.indices, buf.bound_m)
+    plain = (buf.counts, buf.expert_x, buf.expert_scale, xq.to(dev), xs.to(dev), buf.indices,
+             buf.bound_m)
+    rows, scales = [], []
+    for mixed in (False, True):
+        buf.expert_x.view(torch.uint8).zero_()
+        buf.expert_scale.zero_()
+        if quantised_half == "send":
+            ata.dispatch_quant(*quant, do_recv=False)
+        else:
+            ata.dispatch(*plain, do_recv=False)
+        if (quantised_half == "recv") == mixed:
+            ata.dispatch_quant(*quant, do_send=False)
+        else:
+            ata.dispatch(*plain, do_send=False)
+        torch.cuda.synchronize()
+        ata.check_status()
+        rows.append(buf.expert_x.view(torch.uint8).clone())
+        scales.append(buf.expert_scale.clone())
+        ata.combine(buf.out, buf.indices, buf.weights, buf.make_expert_y(), buf.bound_m)
+    assert torch.equal(rows[0], rows[1]) and torch.equal(scales[0], scales[1])
+    assert buf.counts.sum().item() == 600 * cfg.experts_per_token
     ata.destroy()
