@@ -38,9 +38,9 @@ cudaError_t launch_dispatch_tiny(const DispatchArgs& a, bool send, bool recv, in
 cudaError_t launch_dispatch_tiny_multi(const DispatchMulti& args, int nranks, bool send, bool recv,
                                        int grid, cudaStream_t stream);
 
-// Objects whose world is one rank (single_rank.cu): dispatch as one call or as halves, the packed
-// send (a.packed), and combine as one call.  `limit`: blocks at most; the forms that gain from two
-// per SM (whole calls) take more than one per SM where it allows that.
+// Objects whose world is one rank and that have a row_of table (single_rank.cu): dispatch as one
+// call or as halves, the packed send (a.packed), and combine as one call.  `limit`: blocks at most;
+// the forms that gain from two per SM (whole calls) take more than one per SM where it allows that.
 constexpr int kSingleRankBlocksPerSm = 2;
 size_t single_rank_smem_bytes(const A2AParams& p);
 cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, int limit,

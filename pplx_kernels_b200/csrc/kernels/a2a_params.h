@@ -105,8 +105,8 @@ struct A2AParams {
   uint2* row_src;         // [nle][cap] {src_rank | k << 16, src_token} per received row
   uint2* row_of;          // world of one rank: [max_tokens * topk] {local expert, row} of every
                           //     (token, k) of the last dispatch (packed or not), {kNoRow, *}
-                          //     where it has none and for all tokens it did not have; nullptr
-                          //     otherwise
+                          //     where it has none and for all tokens it did not have; nullptr:
+                          //     the general kernels run
   uint32_t* dispatched;   // world of one rank: [2] tokens of the last dispatch of each parity
   Status* status;
   uint64_t timeout_ns;

@@ -161,9 +161,15 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
 
   iter_ = DeviceBuffer<uint32_t>(4);
   recv_count_ = DeviceBuffer<uint32_t>(2 * static_cast<size_t>(params_.nle));
-  // (A world of one rank also keeps where each (token, k) went, behind row_src.)
+  int smem_limit = 0;
+  CUDA_CHECK(cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                    current_device()));
+  // A world of one rank has kernels of its own and keeps where each (token, k) went, behind
+  // row_src.  (Where their tables do not fit a block, thousands of rows per token, it runs the
+  // general ones.)
   const size_t rows = static_cast<size_t>(params_.nle) * params_.cap;
-  const bool single = cfg_.world_size == 1;
+  const bool single = cfg_.world_size == 1 &&
+                      single_rank_smem_bytes(params_) <= static_cast<size_t>(smem_limit);
   row_src_ = DeviceBuffer<uint2>(
       rows + (single ? static_cast<size_t>(params_.max_tokens) * params_.topk : 0));
   status_ = DeviceBuffer<Status>(1);
@@ -206,19 +212,12 @@ AllToAll::AllToAll(const A2AConfig& cfg, std::shared_ptr<SymmetricAllocation> ar
                      : 0;
   num_sms_ = get_sm_count();
   max_blocks_ = static_cast<int>(env_long("PPLX_B200_NUM_SMS", 0));
-  {
-    int smem_limit = 0;
-    CUDA_CHECK(cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin,
-                                      current_device()));
-    const size_t need = single ? std::max(single_rank_smem_bytes(params_), dispatch_smem_bytes(params_))
-                               : dispatch_smem_bytes(params_);
-    PPLX_CHECK(need <= static_cast<size_t>(smem_limit),
-               "num_experts " << cfg_.num_experts << " with world_size " << cfg_.world_size
-                              << " needs " << need
-                              << " bytes of shared memory per block for the dispatch histogram; "
-                                 "the device offers "
-                              << smem_limit);
-  }
+  PPLX_CHECK(dispatch_smem_bytes(params_) <= static_cast<size_t>(smem_limit),
+             "num_experts " << cfg_.num_experts << " with world_size " << cfg_.world_size
+                            << " needs " << dispatch_smem_bytes(params_)
+                            << " bytes of shared memory per block for the dispatch histogram; "
+                               "the device offers "
+                            << smem_limit);
   // Guards after every region of this rank's arena (peers never write there).
   {
     std::vector<uint32_t> pattern(kCanaryBytes / sizeof(uint32_t), kCanaryWord);
@@ -460,7 +459,7 @@ void AllToAll::dispatch_send_packed(const DispatchCall& call, cudaStream_t strea
   NvtxRange range("dispatch_send_packed");
   const DispatchArgs a = make_packed_send_args(call);
   begin(Step::kDispatchSend, false);
-  if (cfg_.world_size == 1) {
+  if (params_.row_of != nullptr) {
     CUDA_CHECK(launch_single_dispatch(a, true, false, block_limit(kSingleRankBlocksPerSm), stream));
     return;
   }
@@ -525,7 +524,7 @@ void AllToAll::dispatch(const DispatchCall& call, SplitMode mode, cudaStream_t s
   const DispatchArgs a = make_dispatch_args(call);
   const bool send = mode != SplitMode::kRecv, recv = mode != SplitMode::kSend;
   begin(send ? Step::kDispatchSend : Step::kDispatchRecv, send && recv);
-  if (cfg_.world_size == 1) {
+  if (params_.row_of != nullptr) {
     CUDA_CHECK(launch_single_dispatch(a, send, recv, block_limit(kSingleRankBlocksPerSm), stream));
     return;
   }
@@ -542,7 +541,7 @@ void AllToAll::combine(const CombineCall& call, SplitMode mode, cudaStream_t str
   CombineArgs a = make_combine_args(call);
   const bool send = mode != SplitMode::kRecv, recv = mode != SplitMode::kSend;
   begin(send ? Step::kCombineSend : Step::kCombineRecv, send && recv);
-  if (cfg_.world_size == 1 && send && recv) {
+  if (params_.row_of != nullptr && send && recv) {
     combine_send_used_lines_ = false;
     CUDA_CHECK(launch_single_combine(a, call.in, call.out, block_limit(kSingleRankBlocksPerSm),
                                      stream));

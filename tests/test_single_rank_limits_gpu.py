@@ -7,7 +7,7 @@ import pplx_kernels_b200 as pk
 from pplx_kernels_b200.ops import _ops
 from pplx_kernels_b200.ops.quant import per_token_block_quant
 from pplx_kernels_b200.utils.testing import MoEConfig
-from pplx_kernels_b200.utils.verify import RankBuffers, verify_dispatch, world_inputs
+from pplx_kernels_b200.utils.verify import RankBuffers, run_local_world, verify_dispatch, world_inputs
 
 pytestmark = pytest.mark.gpu
 
@@ -156,3 +156,10 @@ def test_halves_of_dispatch_and_dispatch_quant(quantised_half):
     assert torch.equal(rows[0], rows[1]) and torch.equal(scales[0], scales[1])
     assert buf.counts.sum().item() == 600 * cfg.experts_per_token
     ata.destroy()
+
+
+def test_object_whose_tables_do_not_fit_one_block():
+    """9000 experts and 7000 rows per token: the kernels of larger worlds take it."""
+    cfg = MoEConfig(num_experts=9000, experts_per_token=7000, hidden_dim=16, max_num_tokens=3)
+    run_local_world(cfg, world=1, dp_size=1, seed=10, num_tokens=3, iterations=2)
+    run_local_world(cfg, world=1, dp_size=1, seed=11, num_tokens=2, split=True)
