@@ -116,6 +116,7 @@ def test_an_expert_named_twice_by_its_tokens(split):
     cfg = MoEConfig(num_experts=4, experts_per_token=3, hidden_dim=64, max_num_tokens=4)
     ata, _, buf = _object(cfg, 5, 4)
     buf.indices = torch.zeros(4, 3, dtype=torch.int32, device=buf.out.device).view(torch.uint32)
+    _ops.sleep_on_stream(0.05)  # both halves are issued before the host can see the failure
     _dispatch(ata, buf, split)
     torch.cuda.synchronize()
     assert buf.counts.tolist() == [12, 0, 0, 0]
