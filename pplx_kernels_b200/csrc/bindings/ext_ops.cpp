@@ -72,7 +72,8 @@ void fake_grouped_gemm(const at::Tensor&, const at::Tensor&, const at::Tensor&, 
 void grouped_gemm_fp8_op(const at::Tensor& xq, const at::Tensor& sa, const at::Tensor& wq,
                          const at::Tensor& sw, const at::Tensor& counts, at::Tensor& out,
                          const std::optional<at::Tensor>& out_scale, bool swiglu_quant,
-                         const std::optional<at::Tensor>& status, bool pow2_scales) {
+                         const std::optional<at::Tensor>& status, bool pow2_scales,
+                         int64_t expected_rows) {
   TORCH_CHECK(xq.is_cuda() && wq.is_cuda() && sa.is_cuda() && sw.is_cuda() && out.is_cuda(),
               "grouped_gemm_fp8: all tensors must be CUDA tensors");
   TORCH_CHECK(xq.element_size() == 1 && wq.element_size() == 1, "xq and wq must be 1-byte (e4m3)");
@@ -95,6 +96,7 @@ void grouped_gemm_fp8_op(const at::Tensor& xq, const at::Tensor& sa, const at::T
   TORCH_CHECK(counts.scalar_type() == at::kInt && counts.numel() == E && counts.is_contiguous(),
               "counts must be a contiguous int32 tensor of [E]");
   Fp8GemmCall c;
+  c.expected_total_rows = expected_rows;
   if (swiglu_quant) {
     TORCH_CHECK(out.element_size() == 1, "with swiglu_quant the output is e4m3");
     TORCH_CHECK(out_scale.has_value() && out_scale->is_cuda() && out_scale->dim() == 3 &&
@@ -145,7 +147,7 @@ void grouped_gemm_fp8_op(const at::Tensor& xq, const at::Tensor& sa, const at::T
 void fake_grouped_gemm_fp8(const at::Tensor&, const at::Tensor&, const at::Tensor&,
                            const at::Tensor&, const at::Tensor&, at::Tensor&,
                            const std::optional<at::Tensor>&, bool,
-                           const std::optional<at::Tensor>&, bool) {}
+                           const std::optional<at::Tensor>&, bool, int64_t) {}
 
 }  // namespace
 
@@ -155,7 +157,8 @@ void register_extension_ops(torch::Library& m) {
   m.impl("grouped_gemm", c10::kCUDA, &grouped_gemm_op);
   m.impl("grouped_gemm", c10::kMeta, &fake_grouped_gemm);
   m.def("grouped_gemm_fp8(Tensor xq, Tensor sa, Tensor wq, Tensor sw, Tensor counts, Tensor! out, "
-        "Tensor!? out_scale, bool swiglu_quant, Tensor!? status, bool pow2_scales=False) -> ()");
+        "Tensor!? out_scale, bool swiglu_quant, Tensor!? status, bool pow2_scales=False, "
+        "int expected_rows=0) -> ()");
   m.impl("grouped_gemm_fp8", c10::kCUDA, &grouped_gemm_fp8_op);
   m.impl("grouped_gemm_fp8", c10::kMeta, &fake_grouped_gemm_fp8);
 }

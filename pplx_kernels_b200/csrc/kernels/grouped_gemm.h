@@ -106,6 +106,7 @@ struct Fp8GemmCall {
   // cores, and the swiglu_quant epilogue emits power-of-two scales in turn.
   bool pow2_scales = false;
   int num_sms = 0;
+  int64_t expected_total_rows = 0;  // hint for the choice of the kernel form; 0 = few
 };
 
 void launch_grouped_gemm_fp8(const Fp8GemmCall& call, cudaStream_t stream);

@@ -67,11 +67,13 @@ struct Control {
   uint32_t abort_flag;
   uint32_t max_tokens;            // widest token tile of this launch
   uint32_t pad;
+  rows::Barriers row_bar;         // kMany
   alignas(16) float scales[kBuffers][128];  // [half * kMaxTokens + token]
   float amax[2][4][64];                     // SwiGLU: [warp group][warp][token of the group's]
   float inv_scale[2][64];
   alignas(16) uint8_t seg[2][2][16][kSegBytes];  // [warp group][alternating][token][column]
 };
+static_assert(sizeof(Control::seg) >= rows::kScratchBytes, "scratch of the form for many rows");
 
 // Tiles of an expert are ordered with the token tile fastest: CTAs that run at the same time
 // share a block of weights in L2.
@@ -199,13 +201,18 @@ __device__ __forceinline__ bool fold_tile(const FoldLoop& f, int own,
   return fold_k_loop<kHalves, kOwn>(f, acc, round);
 }
 
-template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers>
+// kMany: the set-up, then the form for many rows per expert.  (A kernel of its own: with both forms in
+// one, chosen by the row counts on the device, the registers of either were worse and every size was
+// 5 to 10 % slower.)
+template <bool kSwiGLUQuant, bool kFromStaging, bool kToPeers, bool kMany>
 __global__ void __launch_bounds__(kThreads, 1)
     grouped_gemm_fp8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                  const __grid_constant__ CUtensorMap tmap_x64,
                                  const __grid_constant__ CUtensorMap tmap_x16,
                                  const __grid_constant__ Fp8GemmArgs g) {
-  static_assert(!(kFromStaging && kToPeers) && !(kToPeers && kSwiGLUQuant), "unsupported form");
+  static_assert(!(kFromStaging && kToPeers) && !(kToPeers && kSwiGLUQuant) &&
+                    !(kMany && (kSwiGLUQuant || kFromStaging)),
+                "unsupported form");
   constexpr int kHalves = kSwiGLUQuant ? 2 : 1;
   using S = Shape<kHalves>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -240,6 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       tc::mbar_init(&ctl->part_full[b], 2);  // the MMAs, and the scales
       tc::mbar_init(&ctl->part_empty[b], 8);
     }
+    if constexpr (kMany) rows::init_barriers(&ctl->row_bar);
     tc::fence_mbar_init();
     tc::tma_prefetch_desc(&tmap_w);
     tc::tma_prefetch_desc(&tmap_x64);
@@ -322,7 +330,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   // As many stages as the launch's widest token tile leaves room for.
   const uint32_t stage_bytes = S::kWBytes + ctl->max_tokens * kBlockKBytes;
   const uint32_t stages = min(g.ring_bytes / stage_bytes, static_cast<uint32_t>(kMaxStages));
-  if (warp == 0) {
+  if constexpr (kMany) {
+    const rows::Shared shared{ring,       &ctl->row_bar, &ctl->seg[0][0][0][0], peer_stage,
+                              tile_start, rows_of,       abort_flag,            tmem_base};
+    rows::run<kToPeers>(tmap_w, tmap_x64, g, shared);
+  } else if (warp == 0) {
     if (tc::elect_one()) {
       uint32_t stage = 0, phase = 0, pending = 0, pending_phase = 0;
       bool ok = *abort_flag == 0u;

@@ -459,6 +459,7 @@ void AllToAll::dispatch_send_packed(const DispatchCall& call, cudaStream_t strea
   NvtxRange range("dispatch_send_packed");
   const DispatchArgs a = make_packed_send_args(call);
   begin(Step::kDispatchSend, false);
+  expect_rows(call.num_tokens);
   if (params_.row_of != nullptr) {
     CUDA_CHECK(launch_single_dispatch(a, true, false, block_limit(kSingleRankBlocksPerSm), stream));
     return;
@@ -513,7 +514,10 @@ void AllToAll::dispatch_send_packed_group(const std::vector<AllToAll*>& ranks,
   }
   const int n = static_cast<int>(ranks.size());
   const int grid = std::min(ranks[0]->dispatch_grid(max_tokens), std::max(1, ranks[0]->num_sms_ / n));
-  for (AllToAll* r : ranks) r->begin(Step::kDispatchSend, false);
+  for (size_t r = 0; r < ranks.size(); ++r) {
+    ranks[r]->begin(Step::kDispatchSend, false);
+    ranks[r]->expect_rows(calls[r].num_tokens);
+  }
   DispatchMulti multi{};
   for (int r = 0; r < n; ++r) multi.r[r] = args[r];
   CUDA_CHECK(launch_dispatch_multi(multi, n, true, false, grid, stream));
@@ -524,6 +528,7 @@ void AllToAll::dispatch(const DispatchCall& call, SplitMode mode, cudaStream_t s
   const DispatchArgs a = make_dispatch_args(call);
   const bool send = mode != SplitMode::kRecv, recv = mode != SplitMode::kSend;
   begin(send ? Step::kDispatchSend : Step::kDispatchRecv, send && recv);
+  if (send) expect_rows(call.num_tokens);
   if (params_.row_of != nullptr) {
     CUDA_CHECK(launch_single_dispatch(a, send, recv, block_limit(kSingleRankBlocksPerSm), stream));
     return;
@@ -628,6 +633,7 @@ void AllToAll::fused_down_fp8(const FusedFfnFp8Call& f, cudaStream_t stream) {
   c.n_out = params_.hidden_dim;
   c.k = f.inter_dim;
   c.swiglu_quant = false;
+  c.expected_total_rows = expected_rows_;
   c.num_sms = block_limit();
   launch_gemm_fp8_to_peers(c, params_, stream);
 }
@@ -676,7 +682,10 @@ void AllToAll::dispatch_group(const std::vector<AllToAll*>& ranks,
   const int per_rank_limit = std::max(1, ranks[0]->num_sms_ / n);
   grid = std::min(ranks[0]->dispatch_grid(max_tokens), per_rank_limit);
   const bool send = mode != SplitMode::kRecv, recv = mode != SplitMode::kSend;
-  for (AllToAll* r : ranks) r->begin(send ? Step::kDispatchSend : Step::kDispatchRecv, send && recv);
+  for (size_t r = 0; r < ranks.size(); ++r) {
+    ranks[r]->begin(send ? Step::kDispatchSend : Step::kDispatchRecv, send && recv);
+    if (send) ranks[r]->expect_rows(calls[r].num_tokens);
+  }
   DispatchMulti multi{};
   for (int r = 0; r < n; ++r) multi.r[r] = args[r];
   if (ranks[0]->params_.tiny != 0 && !calls[0].quantize) {

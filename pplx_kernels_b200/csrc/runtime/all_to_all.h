@@ -232,6 +232,12 @@ class AllToAll {
   std::vector<size_t> canaries_;
   Step next_ = Step::kDispatchSend;
   bool combine_send_used_lines_ = false;
+  // Rows that this rank's experts get when every rank dispatches as many tokens as this one, evenly
+  // spread: a hint for the fp8 down projection of the fused path.
+  void expect_rows(int num_tokens) {
+    expected_rows_ = static_cast<int64_t>(num_tokens) * params_.topk * params_.num_dp_groups / params_.world;
+  }
+  int64_t expected_rows_ = 0;
   DeviceBuffer<uint64_t> trace_;
   int num_sms_ = 0;
   int max_blocks_ = 0;

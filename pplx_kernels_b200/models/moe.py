@@ -214,7 +214,10 @@ class MoELayerFP8:
                          status=self.gemm_status, pow2_scales=self.pow2_scales)
         grouped_gemm_fp8(self.h, self.h_scale, self.w2_q, self.w2_s, self.counts,
                          out=self.expert_y, status=self.gemm_status,
-                         pow2_scales=self.pow2_scales)
+                         pow2_scales=self.pow2_scales,
+                         # (As in MoELayer.forward: a hint.)
+                         expected_rows=x.size(0) * self.cfg.experts_per_token
+                         * (self.world_size // self.dp_size) // self.world_size)
         self.ata.combine(out, indices, weights, self.expert_y, bound_m)
         return out
 

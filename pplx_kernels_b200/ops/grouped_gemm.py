@@ -57,7 +57,8 @@ def grouped_gemm_reference(x: torch.Tensor, w: torch.Tensor, counts: torch.Tenso
 def grouped_gemm_fp8(xq: torch.Tensor, sa: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor,
                      counts: torch.Tensor, swiglu_quant: bool = False,
                      out: torch.Tensor | None = None, out_scale: torch.Tensor | None = None,
-                     status: torch.Tensor | None = None, pow2_scales: bool = False):
+                     status: torch.Tensor | None = None, pow2_scales: bool = False,
+                     expected_rows: int = 0):
     """Block-scaled fp8 grouped GEMM (tcgen05 ``kind::f8f6f4``, or with ``pow2_scales``
     ``kind::mxf8f6f4.block_scale``).
 
@@ -73,6 +74,10 @@ def grouped_gemm_fp8(xq: torch.Tensor, sa: torch.Tensor, wq: torch.Tensor, sw: t
     ``dispatch_quant(..., pow2=True)``): the tensor cores then apply the scales themselves and the
     whole K range accumulates in tensor memory; the ``swiglu_quant`` epilogue emits power-of-two
     scales in turn.  Mantissa bits of a scale that is not a power of two would be ignored.
+
+    ``expected_rows`` (total valid rows, 0 = few) is a hint: the plain form with fp32 scales has a
+    kernel for many rows per expert, which is taken where it is the faster one.  The numbers of rows
+    are read on the device either way.
     """
     E, rows, _ = xq.shape
     n_out = wq.size(1) // 2 if swiglu_quant else wq.size(1)
@@ -84,7 +89,7 @@ def grouped_gemm_fp8(xq: torch.Tensor, sa: torch.Tensor, wq: torch.Tensor, sw: t
     elif out is None:
         out = torch.empty(E, rows, n_out, dtype=torch.bfloat16, device=xq.device)
     _ops.grouped_gemm_fp8(xq, sa, wq, sw, counts, out, out_scale, swiglu_quant, status,
-                          pow2_scales)
+                          pow2_scales, expected_rows)
     return (out, out_scale) if swiglu_quant else out
 
 
