@@ -7,7 +7,14 @@ import pplx_kernels_b200 as pk
 from pplx_kernels_b200.ops import _ops
 from pplx_kernels_b200.ops.quant import per_token_block_quant
 from pplx_kernels_b200.utils.testing import MoEConfig
-from pplx_kernels_b200.utils.verify import RankBuffers, run_local_world, verify_dispatch, world_inputs
+from pplx_kernels_b200.utils.verify import (
+    EXPERT_GAIN,
+    RankBuffers,
+    run_local_world,
+    verify_combine,
+    verify_dispatch,
+    world_inputs,
+)
 
 pytestmark = pytest.mark.gpu
 
@@ -164,3 +171,57 @@ def test_object_whose_tables_do_not_fit_one_block():
     cfg = MoEConfig(num_experts=9000, experts_per_token=7000, hidden_dim=16, max_num_tokens=3)
     run_local_world(cfg, world=1, dp_size=1, seed=10, num_tokens=3, iterations=2)
     run_local_world(cfg, world=1, dp_size=1, seed=11, num_tokens=2, split=True)
+
+
+def test_dispatch_quant_in_halves_equals_the_whole_call():
+    dev = torch.device("cuda", 0)
+    cfg = MoEConfig(num_experts=16, experts_per_token=4, hidden_dim=1408, max_num_tokens=130,
+                    in_dtype=torch.float8_e4m3fn)
+    ata, _, buf = _object(cfg, 12, 129)
+    x = torch.randn(130, cfg.hidden_dim, generator=torch.Generator().manual_seed(13)).to(torch.bfloat16)
+    got = []
+    for halves in (({},), HALVES):
+        buf.expert_x.view(torch.uint8).zero_()
+        buf.expert_scale.zero_()
+        for kw in halves:
+            ata.dispatch_quant(buf.counts, buf.expert_x, buf.expert_scale, x.to(dev), buf.indices,
+                               buf.bound_m, **kw)
+        torch.cuda.synchronize()
+        ata.check_status()
+        got.append((buf.expert_x.view(torch.uint8).clone(), buf.expert_scale.clone(), buf.counts.clone()))
+        ata.combine(buf.out, buf.indices, buf.weights, buf.make_expert_y(), buf.bound_m)
+    assert all(torch.equal(a, b) for a, b in zip(*got, strict=True))
+    ata.destroy()
+
+
+def test_halves_on_two_streams():
+    """Send halves on one stream, receive halves on another, ordered by events; many passes, so that
+    launches overlap on both streams."""
+    cfg = MoEConfig(num_experts=16, experts_per_token=4, hidden_dim=2048, max_num_tokens=64,
+                    in_dtype=torch.float8_e4m3fn)
+    ata, inputs, buf = _object(cfg, 14, 63)
+    ata.set_timeout_ms(3000)
+    send, recv = torch.cuda.Stream(), torch.cuda.Stream()
+    buf.make_expert_y()
+    d_args = (buf.counts, buf.expert_x, buf.expert_scale, buf.x, buf.x_scale, buf.indices, buf.bound_m)
+    c_args = (buf.out, buf.indices, buf.weights, buf.expert_y, buf.bound_m)
+    torch.cuda.synchronize()
+    for _ in range(50):
+        with torch.cuda.stream(send):
+            ata.dispatch(*d_args, do_recv=False)
+        recv.wait_stream(send)
+        with torch.cuda.stream(recv):
+            ata.dispatch(*d_args, do_send=False)
+            buf.expert_y.copy_((buf.expert_x.to(torch.float32) * EXPERT_GAIN).to(cfg.out_dtype))
+        send.wait_stream(recv)
+        with torch.cuda.stream(send):
+            ata.combine(*c_args, do_recv=False)
+        recv.wait_stream(send)
+        with torch.cuda.stream(recv):
+            ata.combine(*c_args, do_send=False)
+        send.wait_stream(recv)
+    torch.cuda.synchronize()
+    ata.check_status()
+    verify_dispatch(cfg, inputs, 1, 0, buf)
+    verify_combine(cfg, inputs, 0, buf)
+    ata.destroy()

@@ -91,3 +91,22 @@ def test_fused_halves_with_plain_halves(kind, first):
             assert (err <= 0.06 * want.abs() + 0.03 * want.abs().amax()).all(), (n, err.max())
         assert torch.isnan(out[m:].float()).all()
     layer.destroy()
+
+
+@pytest.mark.parametrize("kind", ["fp8", "fp8pow2"])
+def test_fused_layer_with_more_than_64_experts(kind):
+    cfg, m = MoEModelConfig("many", 200, 4, 256, 128), 90
+    dev = torch.device("cuda", 0)
+    layer = MoELayerFP8(cfg, m, init_std=0.05, pow2_scales=kind == "fp8pow2")
+    gen = torch.Generator().manual_seed(6)
+    x = torch.randn(m, cfg.hidden_dim, generator=gen).to(torch.bfloat16).to(dev)
+    idx = routing(m, cfg.num_experts, cfg.experts_per_token, gen)
+    w = torch.softmax(torch.randn(m, cfg.experts_per_token, generator=gen), dim=-1).to(dev)
+    want = moe_reference_fp8(x, idx.to(dev), w, *layer.dequantized_weights(), pow2=kind == "fp8pow2")
+    for _ in range(2):
+        out = layer(x, as_index_tensor(idx, dev), w, fused=True)
+        torch.cuda.synchronize()
+        layer.check_status()
+        err = (out[:m].float() - want).abs()
+        assert (err <= 0.06 * want.abs() + 0.03 * want.abs().amax()).all(), err.max()
+    layer.destroy()
