@@ -39,12 +39,12 @@ cudaError_t launch_dispatch_tiny_multi(const DispatchMulti& args, int nranks, bo
                                        int grid, cudaStream_t stream);
 
 // Objects whose world is one rank and that have a row_of table (single_rank.cu): dispatch as one
-// call or as halves, the packed send (a.packed), and combine as one call.  `limit`: blocks at most;
-// the forms that gain from two per SM (whole calls) take more than one per SM where it allows that.
+// call or as halves, the packed send (a.packed), and combine as one call.  `limit`: blocks at most, for
+// the forms that gain from two per SM (whole calls); `one_per_sm`: for the others.
 constexpr int kSingleRankBlocksPerSm = 2;
 size_t single_rank_smem_bytes(const A2AParams& p);
-cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, int limit,
-                                   cudaStream_t stream);
+cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, int one_per_sm,
+                                   int limit, cudaStream_t stream);
 cudaError_t launch_single_combine(const CombineArgs& a, DType in, DType out, int limit,
                                   cudaStream_t stream);
 

@@ -23,7 +23,8 @@
 // Both are bound by DRAM from a few hundred tokens on and by launch plus two dependent memory
 // round trips below that.  DeepSeek-V3 shape, fp8 in, bf16 out, kernel times before and after:
 // 4096 tokens 215 -> 58 us (272 MB) and 274 -> 110 us (529 MB); 128 tokens 14.2 -> 6.8 and
-// 15.1 -> 6.9 us; 1 token 7.9 -> 5.8 and 6.9 -> 4.4 us.
+// 15.1 -> 6.9 us; 1 token 7.9 -> 5.8 and 6.9 -> 4.4 us.  (Writing the second row table and clearing
+// what an earlier dispatch left has since added 0.1 us to the pass of one token.)
 //
 // Called as separate halves, dispatch stages each TOKEN once (the send half must be done with
 // the caller's tensor) and the receive half spreads it to its rows; a counter of staged units
@@ -184,14 +185,14 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
   uint32_t u = u0 + warp;
   load(u);
 
-  // {iter, comb_iter, dispatched[0], dispatched[1]}; of these, this kernel changes the second and
-  // the third or fourth, which are not used from here.
+  // {iter, comb_iter, dispatched[0], dispatched[1]}.  (This kernel's first block changes comb_iter,
+  // which no other block uses, and the dispatched of its parity.)
   const uint4 state = __ldcg(reinterpret_cast<const uint4*>(p.iter));
   const int parity = static_cast<int>(state.x & 1u);
   const uint32_t dispatched_before = parity != 0 ? state.z : state.w;
   if (blk == 0 && tid == 0) {
     // A new round begins; dispatches started must equal combines finished.
-    const uint32_t iter_now = *p.iter, started = *p.comb_iter;
+    const uint32_t iter_now = state.x, started = state.y;
     if (started != iter_now)
       report_failure(p.status, kOutOfOrder, kPhaseDispatchCounts, 0, iter_now, started, p.rank);
     *p.comb_iter = started + 1u;
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
           if (place.y >= static_cast<uint32_t>(p.cap)) kept = make_uint2(kNoRow, 0u);
         } else if (place.x != kNoRow) {
           p.row_src[static_cast<size_t>(e) * p.cap + place.y] =
-              make_uint2(static_cast<uint32_t>(p.rank) | static_cast<uint32_t>(j % topk) << 16,
+              make_uint2(static_cast<uint32_t>(p.rank) | static_cast<uint32_t>(j - (i - tb) * topk) << 16,
                          static_cast<uint32_t>(i));
         }
         p.row_of[static_cast<size_t>(tb) * topk + j] = kept;
@@ -614,11 +615,10 @@ cudaError_t launch(const void* fn, int grid, size_t smem, void** params, cudaStr
 
 size_t single_rank_smem_bytes(const A2AParams& p) { return dispatch_smem(p); }
 
-cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, int limit,
-                                   cudaStream_t stream) {
+cudaError_t launch_single_dispatch(const DispatchArgs& a, bool send, bool recv, int one_per_sm,
+                                   int limit, cudaStream_t stream) {
   const bool quant = a.quantize != 0;
   const int64_t units = static_cast<int64_t>(a.num_tokens) * chunks_of(a.p, quant);
-  const int one_per_sm = std::min(limit, get_sm_count());
   if (!send) {
     void* params[] = {const_cast<DispatchArgs*>(&a)};
     return launch(reinterpret_cast<const void*>(&single_unstage_kernel), grid_for(units, one_per_sm), 0,

@@ -461,7 +461,8 @@ void AllToAll::dispatch_send_packed(const DispatchCall& call, cudaStream_t strea
   begin(Step::kDispatchSend, false);
   expect_rows(call.num_tokens);
   if (params_.row_of != nullptr) {
-    CUDA_CHECK(launch_single_dispatch(a, true, false, block_limit(kSingleRankBlocksPerSm), stream));
+    CUDA_CHECK(launch_single_dispatch(a, true, false, block_limit(),
+                                      block_limit(kSingleRankBlocksPerSm), stream));
     return;
   }
   CUDA_CHECK(launch_dispatch(a, true, false, dispatch_grid(call.num_tokens), stream));
@@ -530,7 +531,8 @@ void AllToAll::dispatch(const DispatchCall& call, SplitMode mode, cudaStream_t s
   begin(send ? Step::kDispatchSend : Step::kDispatchRecv, send && recv);
   if (send) expect_rows(call.num_tokens);
   if (params_.row_of != nullptr) {
-    CUDA_CHECK(launch_single_dispatch(a, send, recv, block_limit(kSingleRankBlocksPerSm), stream));
+    CUDA_CHECK(launch_single_dispatch(a, send, recv, block_limit(),
+                                      block_limit(kSingleRankBlocksPerSm), stream));
     return;
   }
   if (params_.tiny != 0 && !call.quantize) {
