@@ -213,7 +213,7 @@ class AllToAll:
 
         Two-hop protocol: ranks first exchange their per-expert histograms, then store
         every row at its final, expert-major position in the destination's staging, so
-        that ``fused_up`` can read dense 128-row tiles by TMA.  Follow it with
+        that ``fused_up`` can read dense tiles of an expert's rows by TMA.  Follow it with
         ``fused_up``, ``fused_down`` and ``combine(..., do_send=False)``.
 
         With ``quantize`` (object created with ``hidden_dim_bytes = hidden`` and
@@ -281,6 +281,9 @@ class AllToAll:
         return out
 
     def layout(self) -> dict[str, int]:
+        """Geometry and memory of the object.  ``flag_in_data`` and ``decode_sized_dispatch`` say
+        what the general kernels of an object of this size use; in a world of one rank only the
+        separate halves of combine run those."""
         keys = ("num_local_experts", "num_dp_groups", "rows_per_expert", "region_slots",
                 "slot_bytes", "arena_bytes", "flag_in_data", "line_slot_bytes",
                 "line_combine_slot_bytes", "decode_sized_dispatch", "vmm_arena", "multicast")

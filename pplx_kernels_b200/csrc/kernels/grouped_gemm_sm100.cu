@@ -562,8 +562,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("bar.sync 4, 256;" ::: "memory");
       }
       // A thread's values lie across token rows; each group of 16 tokens passes through shared
-      // memory so that rows leave in 16-byte pieces.  An accumulator that is the only one is
-      // handed back when its last group is in registers (with two of them that was slower).
+      // memory so that rows leave in 16-byte pieces.  The wide form, whose accumulator may be the
+      // only one, hands it back when its last group is in registers; the other, which has two, after
+      // the tile (earlier was slower there).
       const uint32_t t_acc = t_lane + buf * kMmaTokens;
       auto hand_back = [&] {
         tc::tc_fence_before_sync();

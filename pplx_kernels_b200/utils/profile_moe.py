@@ -6,10 +6,11 @@
 
 runs a few forward passes of a one-rank layer whose activations and weights are larger than
 the L2 but hold well under a gigabyte, so that it is the command to put under ``ncu`` with
-``-k regex:<kernel>`` and a small ``-c``: the packed send (``dispatch_kernel``, fused), the
-quantising send (``dispatch_kernel``, fp8 composed), the staging-fed and the peer-storing
-expert GEMMs (``grouped_gemm_kernel`` / ``grouped_gemm_fp8_kernel``, fused) and the combine
-reduction.  Prints CUDA-event times per pass.
+``-k regex:<kernel>`` and a small ``-c``: the one-rank dispatch (``single_dispatch_kernel``), the
+expert GEMMs (``grouped_gemm_kernel``, ``grouped_gemm_fp8_fold_kernel``,
+``grouped_gemm_fp8_mx_kernel``; staging-fed and peer-storing when fused) and combine
+(``single_combine_kernel``, or the reduction of ``combine_kernel`` when fused).  Prints CUDA-event
+times per pass.
 """
 
 from __future__ import annotations
